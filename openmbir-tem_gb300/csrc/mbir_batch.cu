@@ -79,7 +79,7 @@ int Batch::ensure_resources() {
   return MBIR_OK;
 }
 
-// Items grouped by voxel-group shape and modality (one launch each); within a group, colour-0 slices of
+// Items grouped by the kernel they run with, batch_group (one launch each); within a group, colour-0 slices of
 // every engine, then colour-1 slices, engines with the most voxels per slice first so the long
 // items start early.
 int Batch::build_items(const std::vector<SweepArgs>& args) {
@@ -97,7 +97,7 @@ int Batch::build_items(const std::vector<SweepArgs>& args) {
     for (int colour = 0; colour < 2; colour++)
       for (int s : order) {
         const int sh = (args[s].shape >= 1 && args[s].shape <= 4) ? args[s].shape : 4;
-        if (2 * (sh - 1) + (args[s].bf ? 1 : 0) != g) continue;
+        if (batch_group(sh, args[s].bf != 0, table_driven(args[s], eng_[s]->nb())) != g) continue;
         for (int y = colour; y < args[s].g.n_y; y += 2) {
           items_.push_back(make_int2(s, y));
           if (colour == 0) need_[s]++;

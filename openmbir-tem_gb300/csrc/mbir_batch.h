@@ -105,7 +105,7 @@ class Batch {
   double tune_ms_[2] = {0.0, 0.0}, tune_vox_[2] = {0.0, 0.0};  // [512, 256]
   unsigned long long wait_ns_ = 10000000000ull;  // colour-1 wait limit (10 s)
   // launch groups: voxel-group shape (4) x modality (HAADF, bright field), one launch each
-  static constexpr int kShapes = 8;
+  static constexpr int kShapes = kBatchGroups;
   int group_off_[kShapes] = {0};
   int group_cnt_[kShapes] = {0};
   double last_ms_ = 0, total_ms_ = 0;

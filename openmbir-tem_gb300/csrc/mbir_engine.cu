@@ -153,6 +153,7 @@ void Engine::release() {
   dfree(d_hc_lofs_);
   dfree(d_hc_count_);
   hc_valid_.clear();
+  sched_ready_ = false;
   acol_lo_.clear();
   acol_mask_.clear();
   if (ev0_) cudaEventDestroy(static_cast<cudaEvent_t>(ev0_));
@@ -461,6 +462,7 @@ int Engine::build_tables() {
     tab_.t_count[i] = cnt;
     t_rows_ = std::max(t_rows_, cnt);
   }
+  one_row_ = std::all_of(tab_.t_count.begin(), tab_.t_count.end(), [](int c) { return c == 1; });
   // same-colour slices must touch disjoint detector rows
   for (int i = 0; i + 2 < g.n_y; i++)
     if (tab_.t_count[i] > 0 && tab_.t_count[i + 2] > 0 &&
@@ -634,6 +636,9 @@ int Engine::alloc_device() {
     smem_bytes_ = sweep_smem_bytes(g.n_theta, g.n_x, 0, t_rows_, bins_, fp64_, 0);
     smem_sched_bytes_ = sweep_smem_bytes(g.n_theta, g.n_x, 0, t_rows_, bins_, fp64_, 0, true);
   }
+  // table-driven launches: no detector response table
+  smem_table_bytes_ = sweep_smem_bytes(g.n_theta, g.n_x, stage_ ? n_rs_ : 0, t_rows_, -1, fp64_,
+                                       stage_ ? n_sp_ : 0);
   const size_t ns = static_cast<size_t>(g.n_t) * g.n_theta * n_rp_;
   const size_t nh = static_cast<size_t>(g.n_theta) * g.n_r * g.n_t;
   const size_t nv = static_cast<size_t>(g.n_z) * g.n_x * g.n_y;
@@ -946,6 +951,7 @@ int Engine::prepare() {
     const int d = lane_shape(g.n_theta);
     shape_ = d == 0 ? 1 : d + 2;
   }
+  if ((rc = build_acol())) return rc;
   // forward projection + error sinogram (HAADF_ReconstructionEngine.cpp:636-691)
   notify("Starting Forward Projection", 10, MBIR_UPDATE_PROGRESS_VALUE_AND_MESSAGE);
   if ((rc = forward_project())) return rc;
@@ -964,6 +970,57 @@ int Engine::prepare() {
   // everything prepare queued has run: another thread may hand the engine to a batch stream
   if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "prepare sync");
   return MBIR_OK;
+}
+
+// The A-column table of every voxel line (FP32, parallel order), built by the sweep's own
+// arithmetic: the sweeps and projections read it instead of computing the column at every visit.
+// It is optional: without room for it (more than a quarter of the free device memory, or a
+// server that keeps its memory for other requests) the kernels compute the columns.
+int Engine::build_acol() {
+  if (fp64_ || p_.order_mode != MBIR_ORDER_PARALLEL) return MBIR_OK;
+  const bool scheduled = bf_ && p_.nhicd && p_.call_schedule != 1;
+  const Geometry& g = g_;
+  const size_t bytes = acol_bytes();
+  size_t free_b = 0, total_b = 0;
+  if (!scheduled) {  // scheduled calls need the table to be scheduled
+    if (!use_table_ || nb_ != 3 || !one_row_) return MBIR_OK;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4) {
+      cudaGetLastError();
+      return MBIR_OK;
+    }
+  }
+  if (cudaMalloc(&d_acol_, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    d_acol_ = nullptr;
+    return MBIR_OK;
+  }
+  const DevTables tab{d_H_, d_bx_, d_bxd_, d_u0_, d_bz_, d_gw_, d_tfirst_, d_tcount_, d_hval_,
+                      d_lineok_};
+  const int rc = launch_acol_f32(dg_, tab, nb_, d_acol_, static_cast<cudaStream_t>(stream_));
+  return rc ? cuda_check(rc, "A-column table") : MBIR_OK;
+}
+
+size_t Engine::acol_bytes() const {
+  return static_cast<size_t>(g_.n_z) * g_.n_x * g_.n_theta * acol_width(nb_) * sizeof(float4);
+}
+
+// The launch's A-column table and FP32 prior constants
+void Engine::table_args(SweepArgs& a) const {
+  a.acol = d_acol_;
+  a.one_row = one_row_ ? 1 : 0;
+  for (int i = 0; i < 27; i++) a.pf.f[i] = static_cast<float>(flt_.f[i]);
+  a.pf.P = static_cast<float>(flt_.mrf_p);
+  a.pf.Q = static_cast<float>(flt_.mrf_q);
+  a.pf.PQ = a.pf.P - a.pf.Q;
+  a.pf.c = static_cast<float>(flt_.mrf_c);
+  a.pf.sp = static_cast<float>(flt_.sig_p);
+  a.pf.inv_sig_pq = static_cast<float>(flt_.inv_sig_pq);
+  a.pf.alpha = static_cast<float>(flt_.mrf_alpha);
+}
+
+// Dynamic shared memory of a launch that walks the rows
+size_t Engine::walk_smem_bytes(const SweepArgs& a) const {
+  return table_driven(a, nb_) ? smem_table_bytes_ : smem_bytes_;
 }
 
 int Engine::forward_project() {
@@ -1002,11 +1059,12 @@ int Engine::forward_project() {
   a.shape = shape_;
   a.stats = nullptr;
   a.err = d_err_;
+  table_args(a);
   for (int colour = 0; colour < 2; colour++) {
     a.colour = colour;
     a.n_slices = (g.n_y - colour + 1) / 2;
     if (a.n_slices <= 0) continue;
-    int rc = launch_sweep(a, nb_, smem_bytes_, s);
+    int rc = launch_sweep(a, nb_, walk_smem_bytes(a), s);
     if (rc) return cuda_check(rc, "forward projection launch");
   }
   int rc;
@@ -1116,6 +1174,7 @@ int Engine::sweep(int outer, int inner, double* stats4) {
     a.n_rs = stage_ ? n_rs_ : 0;
     a.shape = shape_;
     a.err = d_err_;
+    table_args(a);
     if (bright_field_assisted()) {
       a.bf = 1;
       a.bfa = bfa_sweep_args();
@@ -1127,7 +1186,8 @@ int Engine::sweep(int outer, int inner, double* stats4) {
       a.n_slices = (g.n_y - colour + 1) / 2;
       a.stats = d_stats_ + (colour ? static_cast<size_t>(n0) * kStatSlots : 0);
       if (a.n_slices <= 0) continue;
-      if ((rc = launch_sweep(a, nb_, smem_bytes_, s))) return cuda_check(rc, "ICD sweep launch");
+      if ((rc = launch_sweep(a, nb_, walk_smem_bytes(a), s)))
+        return cuda_check(rc, "ICD sweep launch");
     }
     cudaEventRecord(static_cast<cudaEvent_t>(ev3_), s);
     kernel_timed_ = true;
@@ -1210,6 +1270,7 @@ int Engine::batch_args(int outer, int inner, SweepArgs* out, size_t* smem_needed
   a.n_rs = stage_ ? n_rs_ : 0;
   a.shape = shape_;
   a.err = d_err_;
+  table_args(a);
   a.stats = d_stats_;
   a.colour = 0;
   if (bf_) {  // this call's NHICD list, active mask and magnitude reset, its level schedule
@@ -1222,7 +1283,7 @@ int Engine::batch_args(int outer, int inner, SweepArgs* out, size_t* smem_needed
   }
   a.n_slices = (g.n_y + 1) / 2;
   *out = a;
-  if (smem_needed) *smem_needed = smem_bytes_;
+  if (smem_needed) *smem_needed = walk_smem_bytes(a);
   return MBIR_OK;
 }
 
@@ -1890,6 +1951,7 @@ int Engine::autotune_shape() {
   a.smem_rows = stage_ ? 1 : 0;
   a.n_rs = stage_ ? n_rs_ : 0;
   a.err = d_err_;
+  table_args(a);
   if (bf_) {
     a.bf = 1;
     a.bfa.w = d_w_;
@@ -1915,7 +1977,7 @@ int Engine::autotune_shape() {
       a.colour = colour;
       a.n_slices = (g.n_y - colour + 1) / 2;
       a.stats = d_stats_ + (colour ? static_cast<size_t>(n0) * kStatSlots : 0);
-      if (a.n_slices > 0) rc = launch_sweep(a, nb_, smem_bytes_, s);
+      if (a.n_slices > 0) rc = launch_sweep(a, nb_, walk_smem_bytes(a), s);
     }
     cudaEventRecord(static_cast<cudaEvent_t>(ev1_), s);
     // restore the state for the next candidate (and for the reconstruction itself)

@@ -172,6 +172,8 @@ class Engine {
   double* sweep_stats() const { return d_stat4_; }
   int* error_word() const { return d_err_; }
   int nb() const { return nb_; }
+  // whether prepare may build the A-column table where it is optional (build_acol), and its size
+  void allow_table(bool on) { use_table_ = on; }
   bool fp64() const { return fp64_ != 0; }
   const mbir_params& params() const { return p_; }
   int state() const { return state_; }
@@ -191,6 +193,10 @@ class Engine {
   int bf_run();
   int bf_roi_sum(int kind, double* out);
   int bf_prepare_schedule();                      // A-column table for level-scheduled calls
+  int build_acol();
+  size_t acol_bytes() const;
+  void table_args(SweepArgs& a) const;
+  size_t walk_smem_bytes(const SweepArgs& a) const;
   int host_footprint_bins();                      // acol_lo_, acol_mask_ (once, on demand)
   int bf_schedule(const std::vector<int32_t>& rows, SweepArgs& a);  // the call's levels
   void bf_schedule_readback();                    // queue the device schedule's copy to host
@@ -254,6 +260,10 @@ class Engine {
   bool stage_ = true; // slice fits in shared memory
   size_t smem_bytes_ = 0;
   size_t smem_sched_bytes_ = 0;  // scheduled bright-field calls
+  size_t smem_table_bytes_ = 0;  // table-driven row walks
+  bool use_table_ = true;        // build the A-column table where it is optional
+  bool one_row_ = false;         // every slice meets one detector row
+  bool sched_ready_ = false;     // scheduled calls: schedule storage and table in place
   DevFilter flt_{};
   DevGeom dg_{};
 

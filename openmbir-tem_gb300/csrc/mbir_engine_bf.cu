@@ -150,9 +150,8 @@ int Engine::bf_upload() {
   return MBIR_OK;
 }
 
-// Level-scheduled calls (FP32, parallel order, NHICD): the A-column table of every voxel line
-// (built once on the device by the sweep's own arithmetic) and each entry's first bin and
-// nonzero mask: packed on the device for the device colouring, unpacked on the host
+// Level-scheduled calls (FP32, parallel order, NHICD): each entry's first bin and nonzero mask
+// of the A-column table (build_acol): packed on the device for the device colouring, unpacked on the host
 // (host_footprint_bins) for the host schedules.  Without room for the table the calls walk the
 // rows.
 int Engine::bf_prepare_schedule() {
@@ -161,20 +160,15 @@ int Engine::bf_prepare_schedule() {
   const Geometry& g = g_;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   const size_t nl = static_cast<size_t>(g.n_z) * g.n_x;
-  const size_t n4 = nl * g.n_theta * acol_width(nb_);
-  if (cudaMalloc(&d_acol_, n4 * sizeof(float4)) != cudaSuccess ||
-      cudaMalloc(&d_sched_, nl * sizeof(int)) != cudaSuccess ||
+  if (d_acol_ == nullptr || cudaMalloc(&d_sched_, nl * sizeof(int)) != cudaSuccess ||
       cudaMalloc(&d_lofs_, (nl + 1) * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
-    dfree_any(d_acol_);
     dfree_any(d_sched_);
     dfree_any(d_lofs_);
     return MBIR_OK;
   }
-  const DevTables tab{d_H_, d_bx_, d_bxd_, d_u0_, d_bz_, d_gw_, d_tfirst_, d_tcount_, d_hval_,
-                      d_lineok_};
-  int rc = launch_acol_f32(dg_, tab, nb_, d_acol_, s);
-  if (rc) return cuda_check(rc, "A-column table");
+  sched_ready_ = true;
+  int rc;
   acol_lo_.clear();
   acol_mask_.clear();
   // host schedules: the footprint bins on the host now
@@ -227,7 +221,7 @@ int Engine::bf_prepare_schedule() {
 // The A-column table's first bins and nonzero masks on the host (acol_lo_, acol_mask_), read
 // back from the device table once; used by the host schedules and mbir_get_footprint_bins.
 int Engine::host_footprint_bins() {
-  if (!acol_lo_.empty() || d_acol_ == nullptr) return MBIR_OK;
+  if (!acol_lo_.empty() || !sched_ready_) return MBIR_OK;
   const Geometry& g = g_;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   const size_t nl = static_cast<size_t>(g.n_z) * g.n_x;
@@ -248,7 +242,7 @@ int Engine::host_footprint_bins() {
 // has no A-column table.
 int Engine::bf_schedule(const std::vector<int32_t>& rows, SweepArgs& a) {
   const int kMaxColours = 64 * cwords_;
-  if (d_acol_ == nullptr) return MBIR_OK;
+  if (!sched_ready_) return MBIR_OK;
   const Geometry& g = g_;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   // a colour class holds at most as many lines as the kernel has voxel groups
@@ -613,8 +607,9 @@ int Engine::bf_parallel_args(int iter_nonzero, const DevBF& bfa, SweepArgs* out,
   a.n_rs = stage_ ? n_rs_ : 0;
   a.err = d_err_;
   a.shape = shape_;
+  table_args(a);
   if ((rc = bf_schedule(rows, a))) return rc;
-  size_t smem = a.sched_lines != nullptr ? smem_sched_bytes_ : smem_bytes_;
+  size_t smem = a.sched_lines != nullptr ? smem_sched_bytes_ : walk_smem_bytes(a);
   if (a.sched_lines != nullptr) {
     // room for the schedule itself (offsets and lines) after the layout, when it fits: the
     // class steps then read it from shared memory

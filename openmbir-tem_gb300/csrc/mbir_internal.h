@@ -75,6 +75,13 @@ struct DevFilter {
 
 enum SweepMode : int { kModeICD = 0, kModeProject = 1 };
 
+// The prior's constants in FP32, as the sweep kernels use them: kernel arguments, so that the
+// voxel step reads them from the constant bank.
+struct PriorF {
+  float f[32];           // prior weights by neighbour (27 used)
+  float P, Q, PQ, c, sp, inv_sig_pq, alpha;
+};
+
 // Fixed-point scale of the per-line update magnitudes and the ROI sums accumulated with
 // integer atomics (integer addition is associative, so the sums do not depend on the order in
 // which voxels finish): value = count * 2^-32.
@@ -126,8 +133,16 @@ struct SweepArgs {
   int n_levels;
   const int* sched_count;  // device [2] (lines, levels) written by the colour kernel, or nullptr
                            // (then n_levels holds the level count)
-  const float4* acol;      // [n_z*n_x][n_theta][acol_width(NB)] A-column table (FP32)
+  const float4* acol;      // [n_z*n_x][n_theta][acol_width(NB)] A-column table (FP32) or nullptr
+  int one_row;             // every slice of the engine meets one detector row
+  PriorF pf;               // FP32 prior constants (table-driven sweeps)
 };
+
+// The table-driven FP32 step (table_step in mbir_sweep.cuh) serves three-bin footprints of
+// slices that meet one detector row: every level whose voxels are detector pixels.
+inline bool table_driven(const SweepArgs& a, int nb) {
+  return !a.fp64 && nb == 3 && a.one_row && a.acol != nullptr;
+}
 
 // A-column table entry of one voxel line at one view: the first bin (int bits) and the NB
 // footprint values, padded to whole float4s.
@@ -319,12 +334,21 @@ int launch_sweep_f64(const SweepArgs& a, int nb, size_t smem_bytes, void* stream
 int launch_ref_order_f32(const RefOrderArgs& a, int nb, void* stream);
 // persistent batched sweep (FP32, slices staged or in HBM per series); shape = lane_shape of
 // the largest n_theta in the batch
-// one launch per group = 2 * (voxel-group shape - 1) + bright field; threads: 512 (one CTA per
-// SM) or 256 (two CTAs per SM when the shared memory allows)
+// one launch per group of series that share a kernel; threads: 512 (one CTA per SM) or 256 (two
+// CTAs per SM when the shared memory allows)
+constexpr int kBatchGroups = 16;
+inline int batch_group(int shape, bool bf, bool table) {
+  return 2 * (shape - 1) + (bf ? 1 : 0) + (table ? 8 : 0);
+}
+inline int batch_group_shape(int group) { return (group & 7) / 2 + 1; }
+inline bool batch_group_bf(int group) { return (group & 1) != 0; }
+inline bool batch_group_table(int group) { return group >= 8; }
 int launch_batch_sweep(const BatchArgs& b, int nb, int group, int threads, size_t smem_bytes,
                        int grid,
                        void* stream);
 int launch_batch_sweep_nb3(const BatchArgs& b, int group, int threads, size_t smem_bytes, int grid,
+                           void* stream);
+int launch_batch_sweep_tab(const BatchArgs& b, int group, int threads, size_t smem_bytes, int grid,
                            void* stream);
 int launch_batch_sweep_nb5(const BatchArgs& b, int group, int threads, size_t smem_bytes, int grid,
                            void* stream);

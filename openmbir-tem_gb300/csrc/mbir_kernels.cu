@@ -365,6 +365,7 @@ int launch_sweep_f32_smem(const SweepArgs& a, int nb, size_t smem, void* stream)
 
 int launch_batch_sweep(const BatchArgs& b, int nb, int group, int threads, size_t smem, int grid,
                        void* stream) {
+  if (batch_group_table(group)) return launch_batch_sweep_tab(b, group, threads, smem, grid, stream);
   if (nb == 3) return launch_batch_sweep_nb3(b, group, threads, smem, grid, stream);
   if (nb == 5) return launch_batch_sweep_nb5(b, group, threads, smem, grid, stream);
   return -7;

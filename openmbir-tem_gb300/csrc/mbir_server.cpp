@@ -92,6 +92,13 @@ size_t Server::estimate_bytes(const Request& r) const {
   return rb * (3 * sino + vox) + host_layout + bf + (1u << 20);
 }
 
+// The A-column table of a HAADF request (Engine::build_acol).  It only makes the sweeps faster,
+// so no request is refused for it.
+size_t Server::table_bytes(const Request& r) const {
+  if (r.params.modality == MBIR_MODALITY_BF) return 0;
+  return static_cast<size_t>(r.dims[0]) * r.dims[1] * r.n_theta * 16;
+}
+
 int64_t Server::submit(const mbir_params& p, const float* counts, const float* tilts, int n_theta,
                        int n_r, int n_t, double delta_r, double delta_t, int max_outer,
                        double tol) {
@@ -141,6 +148,14 @@ int Server::admit_locked(std::vector<Request*>& admitted) {
     Request* r = queue_.front();
     if (used_ + static_cast<int64_t>(r->bytes) > budget_) break;  // arrival order: no overtaking
     queue_.pop_front();
+    // tables take at most half of the budget, and none that a queued request's own arrays need
+    const size_t table = table_bytes(*r);
+    int64_t queued = 0;
+    for (const Request* q : queue_) queued += static_cast<int64_t>(q->bytes);
+    const int64_t with = used_ + static_cast<int64_t>(r->bytes + table);
+    const bool room = with + queued <= budget_ && with <= budget_ / 2;
+    r->engine->allow_table(room);
+    if (room) r->bytes += table;
     used_ += static_cast<int64_t>(r->bytes);
     admitted.push_back(r);
     stats_.admitted++;

@@ -66,6 +66,7 @@ class Server {
   void loop();
   void prepare_loop();
   size_t estimate_bytes(const Request& r) const;
+  size_t table_bytes(const Request& r) const;
   int admit_locked(std::vector<Request*>& admitted);
   void retire(Request* r, int code, const std::string& msg);
 

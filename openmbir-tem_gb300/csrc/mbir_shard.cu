@@ -88,7 +88,8 @@ int Engine::sweep_colour(int colour, int outer, int inner, double* st4) {
   a.n_rs = stage_ ? n_rs_ : 0;
   a.shape = shape_;
   a.err = d_err_;
-  size_t smem = smem_bytes_;
+  table_args(a);
+  size_t smem = walk_smem_bytes(a);
   if (bf_) {
     a = slab_args_;
     smem = slab_smem_;
