@@ -1,10 +1,11 @@
-// mbir_batch.cu -- many reconstructions of uneven size advanced together: one persistent,
-// cooperative launch per ICD sweep covers every voxel slice of every engine in the batch
+// mbir_batch.cu -- many reconstructions of uneven size advanced together: one persistent
+// launch per kernel and ICD sweep covers every voxel slice of every engine in the batch
 // (batch_sweep_kernel in mbir_sweep.cuh); gain/offset, variance and cost updates stay per
 // engine.  Each engine keeps its volume, error sinogram and nuisance state resident in HBM.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cstdlib>
 #include <cmath>
 #include <numeric>
@@ -24,6 +25,9 @@ Batch::~Batch() {
   if (d_st4_) cudaFree(d_st4_);
   if (ev0_) cudaEventDestroy(static_cast<cudaEvent_t>(ev0_));
   if (ev1_) cudaEventDestroy(static_cast<cudaEvent_t>(ev1_));
+  if (fork_ev_) cudaEventDestroy(static_cast<cudaEvent_t>(fork_ev_));
+  for (void* e : side_ev_) cudaEventDestroy(static_cast<cudaEvent_t>(e));
+  for (void* t : side_) cudaStreamDestroy(static_cast<cudaStream_t>(t));
   if (stream_) cudaStreamDestroy(static_cast<cudaStream_t>(stream_));
 }
 
@@ -79,6 +83,30 @@ int Batch::ensure_resources() {
   return MBIR_OK;
 }
 
+// Streams of the launches after the first
+int Batch::ensure_side_streams(size_t launches) {
+  if (!fork_ev_) {
+    cudaEvent_t e;
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+      return fail(MBIR_EDEVICE, "batch: event");
+    fork_ev_ = e;
+  }
+  while (side_.size() + 1 < launches) {
+    cudaStream_t t;
+    cudaEvent_t e;
+    if (cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking) != cudaSuccess)
+      return fail(MBIR_EDEVICE, "batch: stream");
+    side_.push_back(t);
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+      cudaStreamDestroy(t);
+      side_.pop_back();
+      return fail(MBIR_EDEVICE, "batch: event");
+    }
+    side_ev_.push_back(e);
+  }
+  return MBIR_OK;
+}
+
 // Items grouped by the kernel they run with, batch_group (one launch each); within a group, colour-0 slices of
 // every engine, then colour-1 slices, engines with the most voxels per slice first so the long
 // items start early.
@@ -96,8 +124,7 @@ int Batch::build_items(const std::vector<SweepArgs>& args) {
     group_off_[g] = static_cast<int>(items_.size());
     for (int colour = 0; colour < 2; colour++)
       for (int s : order) {
-        const int sh = (args[s].shape >= 1 && args[s].shape <= 4) ? args[s].shape : 4;
-        if (batch_group(sh, args[s].bf != 0, table_driven(args[s], eng_[s]->nb())) != g) continue;
+        if (groups_[s] != g) continue;
         for (int y = colour; y < args[s].g.n_y; y += 2) {
           items_.push_back(make_int2(s, y));
           if (colour == 0) need_[s]++;
@@ -121,8 +148,7 @@ int Batch::sweep(const std::vector<std::pair<int, int>>& iters, double* stats) {
   if (rc) return rc;
   const int n = static_cast<int>(eng_.size());
   std::vector<SweepArgs> args(n);
-  size_t smem = 0;
-  int nb = -1, max_theta = 0;
+  int nb = -1;
   int max_optin = 0, per_sm = 0;
   cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_);
   cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device_);
@@ -139,34 +165,31 @@ int Batch::sweep(const std::vector<std::pair<int, int>>& iters, double* stats) {
   const size_t stage_cap = two ? static_cast<size_t>(std::min(max_optin, per_sm / 2 - 1024)) - 2048
                                : static_cast<size_t>(max_optin) - 2048;
   // per-engine set-up (row order, bright-field list, active mask, level schedule) side by side
-  std::vector<size_t> needs(n, 0);
   const std::vector<int> rcs = parallel_for(n, device_, [&](int i) {
     const int outer = iters.empty() ? 0 : iters[i].first;
     const int inner = iters.empty() ? 0 : iters[i].second;
-    return eng_[i]->batch_args(outer, inner, &args[i], &needs[i]);
+    return eng_[i]->batch_args(outer, inner, &args[i]);
   });
   for (int i = 0; i < n; i++)
     if (rcs[i]) return fail(rcs[i], eng_[i]->last_error());
+  // a launch group's shared memory is that of its largest series
+  std::vector<int> groups(n);
+  std::array<size_t, kShapes> smem{};
   for (int i = 0; i < n; i++) {
-    const size_t need = needs[i];
     if (nb < 0) nb = eng_[i]->nb();
     if (eng_[i]->nb() != nb) return fail(MBIR_ENOTSUP, "batch: engines at different voxel sizes");
-    max_theta = std::max(max_theta, args[i].g.n_theta);
-    if (args[i].smem_rows) {
-      if (need > stage_cap) {
-        args[i].smem_rows = 0;
-        args[i].n_rs = 0;
-      } else {
-        smem = std::max(smem, need);
-      }
+    size_t need = eng_[i]->walk_smem_bytes(args[i], stage_cap);
+    if (args[i].smem_rows && need > stage_cap) {
+      args[i].smem_rows = 0;
+      args[i].n_rs = 0;
+      need = eng_[i]->walk_smem_bytes(args[i], stage_cap);
     }
+    const int sh = (args[i].shape >= 1 && args[i].shape <= 4) ? args[i].shape : 4;
+    groups[i] = batch_group(sh, args[i].bf != 0, table_driven(args[i], nb), args[i].smem_rows != 0);
+    smem[groups[i]] = std::max(smem[groups[i]], need);
   }
-  for (int i = 0; i < n; i++)
-    if (!args[i].smem_rows)
-      smem = std::max(smem, sweep_smem_bytes(args[i].g.n_theta, args[i].g.n_x, 0, 1,
-                                             args[i].g.bins, 0, 0));
-  (void)max_theta;
-  if (dirty_ || items_.empty()) {
+  if (dirty_ || items_.empty() || groups != groups_) {
+    groups_ = groups;
     if ((rc = build_items(args))) return rc;
     dirty_ = false;
   }
@@ -181,8 +204,20 @@ int Batch::sweep(const std::vector<std::pair<int, int>>& iters, double* stats) {
   for (int i = 0; i < n; i++) ctr[kShapes + n + i] = need_[i] + (unmet ? 1 : 0);
   cudaMemcpyAsync(d_ctr_, ctr.data(), sizeof(int) * ctr.size(), cudaMemcpyHostToDevice, s);
   cudaEventRecord(static_cast<cudaEvent_t>(ev0_), s);
-  for (int g = 0; g < kShapes; g++) {
-    if (group_cnt_[g] == 0) continue;
+  // one launch per group, side by side, the group with the most work first
+  std::array<double, kShapes> work{};
+  for (int i = 0; i < n; i++)
+    work[groups[i]] += static_cast<double>(args[i].g.n_x) * args[i].g.n_y * args[i].g.n_z *
+                       args[i].g.n_theta;
+  std::vector<int> launch;
+  for (int g = 0; g < kShapes; g++)
+    if (group_cnt_[g] > 0) launch.push_back(g);
+  std::stable_sort(launch.begin(), launch.end(), [&](int x, int y) { return work[x] > work[y]; });
+  if ((rc = ensure_side_streams(launch.size()))) return rc;
+  cudaEventRecord(static_cast<cudaEvent_t>(fork_ev_), s);
+  int launch_rc = 0;
+  for (size_t k = 0; k < launch.size(); k++) {
+    const int g = launch[k];
     BatchArgs b{};
     b.series = d_series_;
     b.items = d_items_ + group_off_[g];
@@ -191,9 +226,17 @@ int Batch::sweep(const std::vector<std::pair<int, int>>& iters, double* stats) {
     b.done = d_ctr_ + kShapes;
     b.need = d_ctr_ + kShapes + n;
     b.wait_ns = wait_ns_;
-    rc = launch_batch_sweep(b, nb, g, threads, smem, grid_, s);
-    if (rc) return fail(MBIR_EDEVICE, std::string("batch sweep launch: ") +
-                                          cudaGetErrorString(cudaGetLastError()));
+    cudaStream_t t = k == 0 ? s : static_cast<cudaStream_t>(side_[k - 1]);
+    if (k > 0) cudaStreamWaitEvent(t, static_cast<cudaEvent_t>(fork_ev_), 0);
+    if (!launch_rc) launch_rc = launch_batch_sweep(b, nb, g, threads, smem[g], grid_, t);
+    if (k > 0) cudaEventRecord(static_cast<cudaEvent_t>(side_ev_[k - 1]), t);
+  }
+  for (size_t k = 1; k < launch.size(); k++)
+    cudaStreamWaitEvent(s, static_cast<cudaEvent_t>(side_ev_[k - 1]), 0);
+  if (launch_rc) {
+    const std::string why = cudaGetErrorString(cudaGetLastError());
+    cudaStreamSynchronize(s);  // the other launches work on the engines' arrays
+    return fail(MBIR_EDEVICE, "batch sweep launch: " + why);
   }
   for (int i = 0; i < n; i++) {
     const int ny = args[i].g.n_y;

@@ -82,6 +82,7 @@ class Batch {
 
  private:
   int ensure_resources();
+  int ensure_side_streams(size_t launches);
   int build_items(const std::vector<SweepArgs>& args);
 
   int device_;
@@ -96,6 +97,9 @@ class Batch {
   double* d_st4_ = nullptr;
   size_t cap_series_ = 0, cap_items_ = 0;
   void* stream_ = nullptr;
+  std::vector<void*> side_;   // streams of the sweep's further launches, with an event each
+  std::vector<void*> side_ev_;
+  void* fork_ev_ = nullptr;
   void* ev0_ = nullptr;
   void* ev1_ = nullptr;
   int grid_ = 0;
@@ -104,7 +108,8 @@ class Batch {
   int tune_sweeps_ = 0;
   double tune_ms_[2] = {0.0, 0.0}, tune_vox_[2] = {0.0, 0.0};  // [512, 256]
   unsigned long long wait_ns_ = 10000000000ull;  // colour-1 wait limit (10 s)
-  // launch groups: voxel-group shape (4) x modality (HAADF, bright field), one launch each
+  // launch groups (batch_group), one launch each; groups_: each series' group
+  std::vector<int> groups_;
   static constexpr int kShapes = kBatchGroups;
   int group_off_[kShapes] = {0};
   int group_cnt_[kShapes] = {0};

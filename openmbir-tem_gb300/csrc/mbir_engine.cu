@@ -501,6 +501,8 @@ int Engine::build_tables() {
         row_entries[z] += nnz;
       }
   });
+  all_lines_ = std::all_of(tab_.line_nonempty.begin(), tab_.line_nonempty.end(),
+                           [](uint8_t v) { return v != 0; });
   footprint_entries_ = 0;
   for (int z = 0; z < g.n_z; z++) footprint_entries_ += row_entries[z];
   return MBIR_OK;
@@ -636,9 +638,6 @@ int Engine::alloc_device() {
     smem_bytes_ = sweep_smem_bytes(g.n_theta, g.n_x, 0, t_rows_, bins_, fp64_, 0);
     smem_sched_bytes_ = sweep_smem_bytes(g.n_theta, g.n_x, 0, t_rows_, bins_, fp64_, 0, true);
   }
-  // table-driven launches: no detector response table
-  smem_table_bytes_ = sweep_smem_bytes(g.n_theta, g.n_x, stage_ ? n_rs_ : 0, t_rows_, -1, fp64_,
-                                       stage_ ? n_sp_ : 0);
   const size_t ns = static_cast<size_t>(g.n_t) * g.n_theta * n_rp_;
   const size_t nh = static_cast<size_t>(g.n_theta) * g.n_r * g.n_t;
   const size_t nv = static_cast<size_t>(g.n_z) * g.n_x * g.n_y;
@@ -658,18 +657,16 @@ int Engine::alloc_device() {
   rc |= dmalloc(&d_tcount_, g.n_y);
   rc |= dmalloc_bytes(&d_hval_, static_cast<size_t>(g.n_y) * kMaxTRows * rb_);
   rc |= dmalloc(&d_rows_, g.n_z);
-  rc |= dmalloc(&d_lineok_, static_cast<size_t>(g.n_z) * g.n_x);
+  // (line flags are also read in whole words)
+  rc |= dmalloc(&d_lineok_, static_cast<size_t>(g.n_z) * g.n_x + 4);
   rc |= dmalloc(&d_cosv_, g.n_theta);
   rc |= dmalloc(&d_sinv_, g.n_theta);
   rc |= dmalloc(&d_Href_, static_cast<size_t>(g.n_theta) * bins_);
   rc |= dmalloc(&d_lines_, static_cast<size_t>(g.n_z) * g.n_x);
   rc |= dmalloc(&d_stats_, static_cast<size_t>((g.n_y + 1) / 2 + 1) * kStatSlots * 2);
   rc |= dmalloc(&d_stat4_, kStatSlots);
-  rc |= dmalloc(&d_mu_, g.n_theta);
-  rc |= dmalloc(&d_gain_, g.n_theta);
   rc |= dmalloc(&d_mu2_, g.n_theta);
   rc |= dmalloc(&d_gain2_, g.n_theta);
-  rc |= dmalloc(&d_wv_, g.n_theta);
   n_chunk_ = std::min(32, std::max(1, g.n_t));
   rc |= dmalloc(&d_partial_, static_cast<size_t>(g.n_theta) * n_chunk_ * 6 +
                                  static_cast<size_t>(prior_blocks_));
@@ -682,7 +679,7 @@ int Engine::alloc_device() {
     rc |= dmalloc(&d_magfx_, nl);
     rc |= dmalloc(&d_mag_, nl);
     rc |= dmalloc(&d_filt_, nl);
-    rc |= dmalloc(&d_active_, nl);
+    rc |= dmalloc(&d_active_, nl + 4);
     rc |= dmalloc(&d_bfpart_, 4096);
     rc |= dmalloc(&d_bfout_, 16);
     rc |= dmalloc(&d_alpha_, g.n_theta);
@@ -693,7 +690,7 @@ int Engine::alloc_device() {
     rc |= dmalloc_bytes(&d_w_, ns * rb_);
     rc |= dmalloc_bytes(&d_bfm_, ns * rb_);
     rc |= dmalloc(&d_sel_, static_cast<size_t>(g.n_t) * g.n_theta * n_sp_);
-    rc |= dmalloc(&d_active_, nl);
+    rc |= dmalloc(&d_active_, nl + 4);
     rc |= dmalloc(&d_stage64_, nh);
   }
   if (rc) return fail(MBIR_ENOMEM, "device allocation failed");
@@ -718,6 +715,7 @@ int Engine::alloc_device() {
   return MBIR_OK;
 }
 
+// gw, mu, gain and wv lie in one block: one copy
 int Engine::upload_views() {
   const int nt = g_.n_theta;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
@@ -1008,6 +1006,7 @@ size_t Engine::acol_bytes() const {
 void Engine::table_args(SweepArgs& a) const {
   a.acol = d_acol_;
   a.one_row = one_row_ ? 1 : 0;
+  a.all_lines = all_lines_ ? 1 : 0;
   for (int i = 0; i < 27; i++) a.pf.f[i] = static_cast<float>(flt_.f[i]);
   a.pf.P = static_cast<float>(flt_.mrf_p);
   a.pf.Q = static_cast<float>(flt_.mrf_q);
@@ -1018,9 +1017,27 @@ void Engine::table_args(SweepArgs& a) const {
   a.pf.alpha = static_cast<float>(flt_.mrf_alpha);
 }
 
-// Dynamic shared memory of a launch that walks the rows
-size_t Engine::walk_smem_bytes(const SweepArgs& a) const {
-  return table_driven(a, nb_) ? smem_table_bytes_ : smem_bytes_;
+// Dynamic shared memory of a launch that walks the rows; table-driven launches take two row
+// caches when they fit in `limit`
+size_t Engine::walk_smem_bytes(const SweepArgs& a, size_t limit) const {
+  const bool staged = a.smem_rows != 0;
+  if (!table_driven(a, nb_))
+    return staged == stage_ ? smem_bytes_
+                            : sweep_smem_bytes(g_.n_theta, g_.n_x, 0, t_rows_, bins_, fp64_, 0);
+  const int n_sp = a.bf ? n_sp_ : 0;
+  const bool project = a.mode == kModeProject;
+  if (limit == 0) limit = static_cast<size_t>(smem_optin_limit()) - 1024;
+  const size_t two =
+      table_smem_bytes(g_.n_theta, g_.n_x, a.n_rs, staged, n_sp, project, 2);
+  return two <= limit ? two
+                      : table_smem_bytes(g_.n_theta, g_.n_x, a.n_rs, staged, n_sp, project, 1);
+}
+
+// Dynamic shared memory of a scheduled bright-field call, without the schedule itself
+size_t Engine::sched_smem_bytes(const SweepArgs& a) const {
+  return table_driven(a, nb_)
+             ? table_smem_bytes(g_.n_theta, 0, a.n_rs, a.smem_rows != 0, n_sp_, false, 1)
+             : smem_sched_bytes_;
 }
 
 int Engine::forward_project() {
@@ -1241,7 +1258,7 @@ ExactArgs Engine::exact_args() {
   return a;
 }
 
-int Engine::batch_args(int outer, int inner, SweepArgs* out, size_t* smem_needed) {
+int Engine::batch_args(int outer, int inner, SweepArgs* out) {
   if (state_ < 2) return fail(MBIR_ESTATE, "batch: engine not prepared");
   if (fp64_ || p_.order_mode != MBIR_ORDER_PARALLEL)
     return fail(MBIR_ENOTSUP, "batch: FP32 parallel-order engines only");
@@ -1283,7 +1300,6 @@ int Engine::batch_args(int outer, int inner, SweepArgs* out, size_t* smem_needed
   }
   a.n_slices = (g.n_y + 1) / 2;
   *out = a;
-  if (smem_needed) *smem_needed = walk_smem_bytes(a);
   return MBIR_OK;
 }
 

@@ -164,9 +164,11 @@ class Engine {
   const Geometry& geometry() const { return g_; }
 
   // Hooks for the batched sweep (mbir_batch.cu).  batch_args fills the sweep arguments of this
-  // engine's next parallel-order sweep (uploading its row order) and reports the shared memory
-  // a staged slice needs; batch_finish records a sweep that ran inside a batch.
-  int batch_args(int outer, int inner, SweepArgs* out, size_t* smem_needed);
+  // engine's next parallel-order sweep (uploading its row order); walk_smem_bytes is the shared
+  // memory of its slices as the arguments stage them (two row caches only within `limit`);
+  // batch_finish records a sweep that ran inside a batch.
+  int batch_args(int outer, int inner, SweepArgs* out);
+  size_t walk_smem_bytes(const SweepArgs& a, size_t limit = 0) const;
   int batch_finish(int outer, int inner, const double* st4, double ms);
   double* slice_stats() const { return d_stats_; }
   double* sweep_stats() const { return d_stat4_; }
@@ -196,7 +198,7 @@ class Engine {
   int build_acol();
   size_t acol_bytes() const;
   void table_args(SweepArgs& a) const;
-  size_t walk_smem_bytes(const SweepArgs& a) const;
+  size_t sched_smem_bytes(const SweepArgs& a) const;
   int host_footprint_bins();                      // acol_lo_, acol_mask_ (once, on demand)
   int bf_schedule(const std::vector<int32_t>& rows, SweepArgs& a);  // the call's levels
   void bf_schedule_readback();                    // queue the device schedule's copy to host
@@ -260,9 +262,9 @@ class Engine {
   bool stage_ = true; // slice fits in shared memory
   size_t smem_bytes_ = 0;
   size_t smem_sched_bytes_ = 0;  // scheduled bright-field calls
-  size_t smem_table_bytes_ = 0;  // table-driven row walks
   bool use_table_ = true;        // build the A-column table where it is optional
   bool one_row_ = false;         // every slice meets one detector row
+  bool all_lines_ = false;       // no voxel line's A-column is empty
   bool sched_ready_ = false;     // scheduled calls: schedule storage and table in place
   DevFilter flt_{};
   DevGeom dg_{};

@@ -135,10 +135,11 @@ struct SweepArgs {
                            // (then n_levels holds the level count)
   const float4* acol;      // [n_z*n_x][n_theta][acol_width(NB)] A-column table (FP32) or nullptr
   int one_row;             // every slice of the engine meets one detector row
+  int all_lines;           // no voxel line's A-column is empty
   PriorF pf;               // FP32 prior constants (table-driven sweeps)
 };
 
-// The table-driven FP32 step (table_step in mbir_sweep.cuh) serves three-bin footprints of
+// The table-driven FP32 kernels (mbir_table.cuh) serve three-bin footprints of
 // slices that meet one detector row: every level whose voxels are detector pixels.
 inline bool table_driven(const SweepArgs& a, int nb) {
   return !a.fp64 && nb == 3 && a.one_row && a.acol != nullptr;
@@ -320,6 +321,11 @@ int launch_exact_view_sums(const ExactArgs& a, int kind, const double* y, const 
 // launchers (mbir_kernels.cu); fp64 selects Real = double for the void* arrays
 int launch_sweep(const SweepArgs& a, int nb, size_t smem_bytes, void* stream);
 int launch_ref_order(const RefOrderArgs& a, int nb, void* stream);
+// table-driven launches (mbir_table.cuh) and their shared memory; n_x = 0 for scheduled calls
+int launch_table_haadf(const SweepArgs& a, size_t smem_bytes, void* stream);
+int launch_table_bf(const SweepArgs& a, size_t smem_bytes, void* stream);
+size_t table_smem_bytes(int n_theta, int n_x, int n_rs, bool stage, int n_sp, bool project,
+                        int nbuf);
 // sched: the layout of a scheduled bright-field call (smaller: no response table or row lists)
 size_t sweep_smem_bytes(int n_theta, int n_x, int n_rs, int t_rows, int bins, int fp64,
                         int n_sp, bool sched = false);
@@ -336,20 +342,23 @@ int launch_ref_order_f32(const RefOrderArgs& a, int nb, void* stream);
 // the largest n_theta in the batch
 // one launch per group of series that share a kernel; threads: 512 (one CTA per SM) or 256 (two
 // CTAs per SM when the shared memory allows)
-constexpr int kBatchGroups = 16;
-inline int batch_group(int shape, bool bf, bool table) {
-  return 2 * (shape - 1) + (bf ? 1 : 0) + (table ? 8 : 0);
+constexpr int kBatchGroups = 24;  // shapes x modality, x 3: general, table-driven in HBM, staged
+inline int batch_group(int shape, bool bf, bool table, bool staged) {
+  return 2 * (shape - 1) + (bf ? 1 : 0) + (table ? (staged ? 16 : 8) : 0);
 }
 inline int batch_group_shape(int group) { return (group & 7) / 2 + 1; }
 inline bool batch_group_bf(int group) { return (group & 1) != 0; }
 inline bool batch_group_table(int group) { return group >= 8; }
+inline bool batch_group_staged(int group) { return group >= 16; }
 int launch_batch_sweep(const BatchArgs& b, int nb, int group, int threads, size_t smem_bytes,
                        int grid,
                        void* stream);
 int launch_batch_sweep_nb3(const BatchArgs& b, int group, int threads, size_t smem_bytes, int grid,
                            void* stream);
-int launch_batch_sweep_tab(const BatchArgs& b, int group, int threads, size_t smem_bytes, int grid,
-                           void* stream);
+int launch_batch_table_haadf(const BatchArgs& b, int group, int threads, size_t smem_bytes,
+                             int grid, void* stream);
+int launch_batch_table_bf(const BatchArgs& b, int group, int threads, size_t smem_bytes, int grid,
+                          void* stream);
 int launch_batch_sweep_nb5(const BatchArgs& b, int group, int threads, size_t smem_bytes, int grid,
                            void* stream);
 int launch_ref_order_f64(const RefOrderArgs& a, int nb, void* stream);

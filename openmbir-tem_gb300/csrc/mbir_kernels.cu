@@ -365,7 +365,9 @@ int launch_sweep_f32_smem(const SweepArgs& a, int nb, size_t smem, void* stream)
 
 int launch_batch_sweep(const BatchArgs& b, int nb, int group, int threads, size_t smem, int grid,
                        void* stream) {
-  if (batch_group_table(group)) return launch_batch_sweep_tab(b, group, threads, smem, grid, stream);
+  if (batch_group_table(group))
+    return batch_group_bf(group) ? launch_batch_table_bf(b, group, threads, smem, grid, stream)
+                                 : launch_batch_table_haadf(b, group, threads, smem, grid, stream);
   if (nb == 3) return launch_batch_sweep_nb3(b, group, threads, smem, grid, stream);
   if (nb == 5) return launch_batch_sweep_nb5(b, group, threads, smem, grid, stream);
   return -7;
@@ -373,6 +375,8 @@ int launch_batch_sweep(const BatchArgs& b, int nb, int group, int threads, size_
 
 int launch_sweep(const SweepArgs& a, int nb, size_t smem, void* stream) {
   if (a.fp64) return launch_sweep_f64(a, nb, smem, stream);
+  if (table_driven(a, nb))
+    return a.bf ? launch_table_bf(a, smem, stream) : launch_table_haadf(a, smem, stream);
   return a.smem_rows ? launch_sweep_f32_smem(a, nb, smem, stream)
                      : launch_sweep_f32_hbm(a, nb, smem, stream);
 }

@@ -310,9 +310,12 @@ __device__ __forceinline__ unsigned long long fix32<float>(float v) {
   // integer part and 32-bit fraction converted apart (both exact up to the same rounding): a
   // 64-bit conversion runs on the FP64 pipe, 16 cycles of the SM per warp
   const float a = fabsf(v);
-  if (!(a < 4294967296.0f)) return __float2ull_rn(a * 4294967296.0f);
-  const unsigned hi = __float2uint_rz(a);
-  const unsigned lo = __float2uint_rn((a - __uint2float_rz(hi)) * 4294967296.0f);
+  unsigned hi = __float2uint_rz(a);
+  unsigned lo = __float2uint_rn((a - __uint2float_rz(hi)) * 4294967296.0f);
+  if (!(a < 4294967296.0f)) {  // saturated, NaN as the 64-bit conversion gives it
+    hi = a != a ? 0x80000000u : 0xffffffffu;
+    lo = a != a ? 0u : 0xffffffffu;
+  }
   return (static_cast<unsigned long long>(hi) << 32) | lo;
 }
 
@@ -703,315 +706,6 @@ __device__ __forceinline__ void group_step(const SliceCtx<Real>& c, int z, int x
   }
 }
 
-// ---- table-driven step (FP32, three-bin footprints, one detector row per slice) ------------
-// The same voxel update as group_step, operation for operation, with everything that does not
-// depend on the voxel taken out of it.
-//
-// What bounds it: the sweep is a chain of class steps, each a serial chain of one warp's
-// instructions (group_step issued ~1290 per voxel pair, ~1250 with the A-column table, at about
-// one per 6 cycles), while the detector rows stay in shared memory.  So the step is written for
-// few instructions: the A-column comes from the engine's table (16 bytes per view instead of ~60
-// instructions), per-view constants and offsets stay in registers for the whole slice, the
-// prior's constants are kernel arguments, footprint entries are read unconditionally and only
-// their sums and stores are predicated, and the Bragg selector's rejected entries (rare) take a
-// separate path.
-template <int G, int VPL, bool BF>
-struct TabCtx {
-  const float4* acol;         // A-column table, at this lane's first view
-  float* es;                  // error rows of the slice
-  int eoff[VPL];              // this lane's views' rows in es (0 without a view)
-  float gx[VPL];              // gain
-  float gw[BF ? 1 : VPL];     // weight (HAADF)
-  const float* bw;            // bright field: weights and selector rows of the slice
-  uint8_t* bs;
-  int woff[BF ? VPL : 1], soff[BF ? VPL : 1];
-  float bt, bdt;
-  unsigned long long* mag_fx;
-  float hh;                   // t-response
-  float* vol_y;               // the slice's plane
-  const float* cache;         // neighbour rows of the z-row walked (nullptr: scheduled calls)
-  float* cache_mid;
-  int noff[2];                // this lane's neighbours: offset in the cache or in the volume
-  int ndz[2], ndx[2];
-  bool nok[2];                // the lane has that neighbour and its y lies in the volume
-  bool nco[2];                // read past L1: another CTA of the launch writes that plane
-  float nf[2];                // prior weight
-};
-
-template <int G, int VPL, bool STAGE, bool BF>
-__device__ __forceinline__ void tab_ctx(TabCtx<G, VPL, BF>& c, const SweepArgs& A, int y,
-                                        float* es, int rs, const float* bw, uint8_t* bs, int bs_rs,
-                                        float hh, const float* cache, bool sched, bool coherent,
-                                        int lane) {
-  const DevGeom& g = A.g;
-  const int gl = lane & (G - 1);
-  const int plane = g.n_z * g.n_x;
-  const float2* ggw = static_cast<const float2*>(A.tab.gw);
-  c.acol = A.acol + gl;
-  c.es = es;
-  c.bw = bw;
-  c.bs = bs;
-#pragma unroll
-  for (int i = 0; i < VPL; ++i) {
-    const int v = gl + G * i;
-    const bool ok = v < g.n_theta;
-    const float2 gw = ok ? ggw[v] : make_float2(0.f, 0.f);
-    c.eoff[i] = ok ? v * rs : 0;
-    c.gx[i] = gw.x;
-    if constexpr (BF) {
-      c.woff[i] = ok ? v * g.n_rp : 0;
-      c.soff[i] = ok ? v * bs_rs : 0;
-    } else {
-      c.gw[i] = gw.y;
-    }
-  }
-  c.bt = c.bdt = 0.f;
-  c.mag_fx = nullptr;
-  if constexpr (BF) {
-    c.bt = static_cast<float>(A.bfa.bragg_t);
-    c.bdt = static_cast<float>(A.bfa.bragg_dt);
-    c.mag_fx = A.bfa.mag_fx;
-  }
-  c.hh = hh;
-  c.vol_y = static_cast<float*>(A.x) + static_cast<size_t>(y) * plane;
-  c.cache = sched ? nullptr : cache;
-  c.cache_mid = const_cast<float*>(cache) + 4 * g.n_x;
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int k = gl + G * i;
-    const int dy = k / 9 - 1, dz = (k / 3) % 3 - 1, dx = k % 3 - 1;
-    c.ndz[i] = dz;
-    c.ndx[i] = dx;
-    c.nok[i] = k < 27 && k != 13 && y + dy >= 0 && y + dy < g.n_y;
-    c.nco[i] = coherent && dy != 0;
-    c.noff[i] = sched ? dy * plane + dz * g.n_x + dx : ((dy + 1) * 3 + dz + 1) * g.n_x + dx;
-    c.nf[i] = A.pf.f[k < 27 ? k : 0];
-  }
-}
-
-// rho'(d)/d, the FP32 qggmrf_coef with the kernel's constants
-__device__ __forceinline__ float qggmrf_coef_tab(const PriorF& q, float d0) {
-  const float ad = fabsf(d0);
-  const float t1 = __powf(ad, q.PQ) * q.inv_sig_pq;
-  const float t3 = q.c + t1;
-  float r = __fdividef(q.P * q.c + q.Q * t1, t3 * t3 * q.sp);
-  if (q.P != 2.f) r *= __powf(ad, q.P - 2.f);
-  return d0 == 0.f ? q.P / (q.sp * q.c) : r;
-}
-
-// One voxel (z, x) of the slice per group of G lanes; all 32 lanes of the warp call it together.
-// SCHED: a scheduled call (neighbours from the volume); otherwise a row of the walk (neighbours
-// from the cache).
-template <int G, int VPL, bool STAGE, bool BF, bool SCHED>
-__device__ __forceinline__ void table_step(const SweepArgs& A, const TabCtx<G, VPL, BF>& c, int z,
-                                           int x, bool active, int lane, bool zs,
-                                           GroupAcc& acc) {
-  constexpr int NB = 3, NNB = (27 + G - 1) / G;
-  const int gl = lane & (G - 1);
-  const int n_x = A.g.n_x, n_theta = A.g.n_theta;
-  const int line = z * n_x + x;
-  float4 aq[VPL];
-  {
-    const float4* ac = c.acol + static_cast<size_t>(line) * n_theta;
-#pragma unroll
-    for (int i = 0; i < VPL; ++i)
-      aq[i] = (active && gl + G * i < n_theta) ? __ldg(ac + G * i)
-                                               : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  // neighbours (UpdateVoxels.cpp:283-306); V last, so that a lane's loads are in flight together
-  float nb[NNB];
-  bool nv_ok[NNB];
-  bool pos = false;
-#pragma unroll
-  for (int i = 0; i < NNB; ++i) {
-    nv_ok[i] = c.nok[i] && static_cast<unsigned>(x + c.ndx[i]) < static_cast<unsigned>(n_x) &&
-               static_cast<unsigned>(z + c.ndz[i]) < static_cast<unsigned>(A.g.n_z);
-    nb[i] = 0.f;
-    if (nv_ok[i]) {
-      if constexpr (SCHED) {
-        const float* src = c.vol_y + (line + c.noff[i]);
-        nb[i] = c.nco[i] ? __ldcg(src) : *src;
-      } else {
-        nb[i] = c.cache[c.noff[i] + x];
-      }
-    }
-    pos |= nb[i] > 0.f;
-  }
-  const float V = SCHED ? c.vol_y[line] : c.cache_mid[x];
-  bool live = active;
-  if (zs) {  // zero skipping at the visit; the ballot runs on all 32 lanes
-    const bool any_pos = group_any<G>(pos, lane);
-    if (V == 0.f && !any_pos) {
-      if (active && gl == 0) acc.v[2] += 1;
-      live = false;
-    }
-    if (!__any_sync(kFull, live)) return;
-  }
-
-  // footprint entries, all in flight together
-  float ev[VPL][NB];
-  float wv[BF ? VPL : 1][NB];
-  unsigned sv[BF ? VPL : 1][NB];
-#pragma unroll
-  for (int i = 0; i < VPL; ++i) {
-    const int j = __float_as_int(aq[i].x);
-    const float* er = c.es + (c.eoff[i] + j);
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      const bool p = f4_at(aq[i], b + 1) > 0.f;
-      if constexpr (STAGE) {
-        ev[i][b] = er[b];
-      } else {
-        ev[i][b] = 0.f;
-        if (p) ev[i][b] = er[b];
-      }
-      if constexpr (BF) {
-        wv[i][b] = 0.f;
-        if (p) wv[i][b] = __ldg(c.bw + (c.woff[i] + j) + b);
-        if constexpr (STAGE) {
-          sv[i][b] = c.bs[c.soff[i] + j + b];
-        } else {
-          sv[i][b] = 1;
-          if (p) sv[i][b] = c.bs[c.soff[i] + j + b];
-        }
-      }
-    }
-  }
-
-  // QGGMRF surrogate sums (QGGMRF_Functions.cpp:153-206): arithmetic under the loads above
-  float s1 = 0.f, s2 = 0.f, lo = 0.f, hi = 0.f;
-#pragma unroll
-  for (int i = 0; i < NNB; ++i) {
-    const float tc = c.nf[i] * qggmrf_coef_tab(A.pf, V - nb[i]);
-    if (nv_ok[i]) {
-      s1 += tc * nb[i];
-      s2 += tc;
-    }
-    lo = nb[i] < lo ? nb[i] : lo;
-    hi = nb[i] > hi ? nb[i] : hi;
-  }
-
-  // theta1 / theta2 (UpdateVoxels.cpp:343-369; BF: BFForwardModel.cpp:851-892)
-  float t1 = 0.f, t2 = 0.f;
-  bool rejected = false;
-  if constexpr (BF) {
-#pragma unroll
-    for (int i = 0; i < VPL; ++i)
-#pragma unroll
-      for (int b = 0; b < NB; ++b) rejected |= f4_at(aq[i], b + 1) > 0.f && sv[i][b] == 0;
-  }
-  if (!BF || !__any_sync(kFull, rejected)) {
-#pragma unroll
-    for (int i = 0; i < VPL; ++i)
-#pragma unroll
-      for (int b = 0; b < NB; ++b) {
-        const float a = f4_at(aq[i], b + 1);
-        const float w = BF ? wv[BF ? i : 0][b] : c.gw[BF ? 0 : i];
-        const float pe = c.gx[i] * a * c.hh;
-        const float x2 = pe * pe * w, x1 = ev[i][b] * pe * w;
-        if (a > 0.f) {
-          t2 += x2;
-          t1 += x1;
-        }
-      }
-  } else if constexpr (BF) {
-    // entries that the selector rejects count with weight delta T / (|e| sqrt(w))
-#pragma unroll
-    for (int i = 0; i < VPL; ++i)
-#pragma unroll
-      for (int b = 0; b < NB; ++b) {
-        const float a = f4_at(aq[i], b + 1);
-        const float w = wv[i][b];
-        const float pe = c.gx[i] * a * c.hh;
-        if (a > 0.f) {
-          if (sv[i][b]) {
-            t2 += pe * pe * w;
-            t1 += ev[i][b] * pe * w;
-          } else {
-            const float qc = c.bdt / (fabsf(ev[i][b]) * sqrtf(w));
-            t2 += qc * (pe * pe * w);
-            t1 += qc * (ev[i][b] * pe * w);
-          }
-        }
-      }
-  }
-  const float theta1 = -group_sum<G>(t1);
-  const float theta2 = group_sum<G>(t2);
-  lo = group_min<G>(lo);
-  hi = group_max<G>(hi);
-  s1 = group_sum<G>(s1);
-  s2 = group_sum<G>(s2);
-  // bracket, surrogate minimum, positivity (UpdateVoxels.cpp:47-63, 372-400)
-  if (theta2 != 0.f) {
-    const float cand = V - theta1 / theta2;
-    lo = lo > cand ? cand : lo;
-    hi = hi < cand ? cand : hi;
-  }
-  const float u = (s1 + theta2 * V - theta1) / (s2 + theta2);
-  float nv = V + A.pf.alpha * (u - V);
-  nv = (nv < lo) ? lo : ((nv > hi) ? hi : nv);
-  if (nv < 0.f) nv = 0.f;
-  const float dlt = nv - V;
-  if (!live) return;
-  // error-sinogram scatter (UpdateVoxels.cpp:423-449); BF re-evaluates the selector of every
-  // footprint entry even when the voxel did not change (BFForwardModel.cpp:898-932)
-  if (BF || dlt != 0.f) {
-#pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const int j = __float_as_int(aq[i].x);
-      float* er = c.es + (c.eoff[i] + j);
-#pragma unroll
-      for (int b = 0; b < NB; ++b) {
-        const float a = f4_at(aq[i], b + 1);
-        const float ne = ev[i][b] - c.gx[i] * (a * c.hh * dlt);
-        if (a > 0.f) {
-          er[b] = ne;
-          if constexpr (BF)
-            c.bs[c.soff[i] + j + b] = bragg_selected<float>(ne, wv[i][b], c.bt);
-        }
-      }
-    }
-  }
-  if (gl == 0) {
-    c.vol_y[line] = nv;
-    if constexpr (!SCHED) c.cache_mid[x] = nv;
-    const DevGeom& g = A.g;
-    if (x >= g.roi_x0 && x <= g.roi_x1 && z >= g.roi_z0 && z <= g.roi_z1) {
-      acc.v[0] += fix32<float>(dlt);
-      acc.v[1] += fix32<float>(V);
-    }
-    acc.v[3] += 1;
-    if constexpr (BF) {
-      if (c.mag_fx != nullptr && dlt != 0.f) atomicAdd(c.mag_fx + line, fix32<float>(dlt));
-    }
-  }
-}
-
-// Projection of one voxel per group: its footprint added to the slice's rows
-// (HAADF_ReconstructionEngine.cpp:636-691).
-template <int G, int VPL, bool STAGE, bool BF>
-__device__ __forceinline__ void table_project(const SweepArgs& A, const TabCtx<G, VPL, BF>& c,
-                                              int z, int x, bool active, int lane) {
-  const int gl = lane & (G - 1);
-  const int n_theta = A.g.n_theta;
-  const float V = c.cache_mid[x];
-  const float4* ac = c.acol + static_cast<size_t>(z * A.g.n_x + x) * n_theta;
-  float4 aq[VPL];
-#pragma unroll
-  for (int i = 0; i < VPL; ++i)
-    aq[i] = (active && V != 0.f && gl + G * i < n_theta) ? __ldg(ac + G * i)
-                                                         : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int i = 0; i < VPL; ++i) {
-    float* er = c.es + (c.eoff[i] + __float_as_int(aq[i].x));
-#pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      const float a = f4_at(aq[i], b + 1);
-      if (a > 0.f) er[b] += c.gx[i] * (a * c.hh * V);
-    }
-  }
-}
-
 struct SmemLayout {
   size_t bar, ctl, stats, rb, bx, bxd, gw, H, hv, list, cls, okr, lv, flat, gofs, bits, cache, es,
       sel, total;
@@ -1037,6 +731,8 @@ __host__ __device__ inline SmemLayout smem_layout(int n_theta, int n_x, int n_rs
   o += 16;
   L.ctl = o;  // class counters [2], zero-skip counter
   o += 16;
+  L.stats = o;
+  o += sizeof(unsigned long long) * kMaxGroups * kStatSlots;
   L.rb = o;
   o = align_up(o + 8 * static_cast<size_t>(n_theta), 16);
   L.bx = o;
@@ -1070,11 +766,6 @@ __host__ __device__ inline SmemLayout smem_layout(int n_theta, int n_x, int n_rs
   o = align_up(o, 16);
   L.sel = o;
   if (stage && n_sp > 0) o += static_cast<size_t>(t_rows) * n_theta * n_sp;
-  o = align_up(o, 16);
-  // after the rows: table_step reads the two entries before and after a view's row whether or
-  // not the footprint has them, and those reads stay inside the layout
-  L.stats = o;
-  o += sizeof(unsigned long long) * kMaxGroups * kStatSlots;
   L.total = align_up(o, 16);
   return L;
 }
@@ -1091,8 +782,7 @@ __host__ __device__ inline SmemLayout smem_layout(int n_theta, int n_x, int n_rs
 // slices); `coherent` makes neighbour-row loads bypass L1 (needed when other CTAs of the same
 // launch write neighbouring slices).  Writes the slice's four statistics to stat_out when it
 // is not null.  Returns false when a bounded wait gave up (A.err is set).
-// TAB: the table-driven step (table_step); otherwise group_step.
-template <typename Real, int NB, int G, int VPL, bool STAGE, bool BF, bool TAB>
+template <typename Real, int NB, int G, int VPL, bool STAGE, bool BF>
 __device__ __forceinline__ bool run_slice(const SweepArgs& A, int y, unsigned char* smem,
                                           uint32_t& phase, bool coherent, double* stat_out) {
   using R2 = typename V2<Real>::type;
@@ -1106,9 +796,8 @@ __device__ __forceinline__ bool run_slice(const SweepArgs& A, int y, unsigned ch
   const int n_sp = BF ? A.bfa.n_sp : 0;
   const bool sched_layout = BF && std::is_same<Real, float>::value && A.sched_lines != nullptr &&
                             A.acol != nullptr && A.mode != kModeProject;
-  // table-driven slices have no detector response table (bins = -1)
-  const SmemLayout L = smem_layout(g.n_theta, g.n_x, A.n_rs, tcount, TAB ? -1 : g.bins, STAGE,
-                                   sizeof(Real), n_sp, sched_layout);
+  const SmemLayout L = smem_layout(g.n_theta, g.n_x, A.n_rs, tcount, g.bins, STAGE, sizeof(Real),
+                                   n_sp, sched_layout);
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L.bar);
   unsigned* ctl = reinterpret_cast<unsigned*>(smem + L.ctl);
   unsigned long long* sstat = reinterpret_cast<unsigned long long*>(smem + L.stats);
@@ -1129,20 +818,18 @@ __device__ __forceinline__ bool run_slice(const SweepArgs& A, int y, unsigned ch
 
   __shared__ PriorConst<Real> s_pc;
   __shared__ Real s_qf[27];
-  if constexpr (!TAB) {
-    if (tid == 0) s_pc = prior_const<Real>(A.flt, A.g);
-    if (tid < 27) s_qf[tid] = static_cast<Real>(A.flt.f[tid]);
-    if (!sched_layout)  // scheduled calls read the A-column from its table
-      for (int i = tid; i < g.n_theta * (g.bins + 1); i += nthreads) sH[i] = gH[i];
-    for (int v = tid; v < g.n_theta; v += nthreads) {
-      if (kF32)
-        sbx[v] = A.tab.bx[v];
-      else
-        sbxd[v] = A.tab.bxd[v];
-      sgw[v] = ggw[v];
-    }
-    if (tid < kMaxTRows) shv[tid] = ghv[y * kMaxTRows + tid];
+  if (tid == 0) s_pc = prior_const<Real>(A.flt, A.g);
+  if (tid < 27) s_qf[tid] = static_cast<Real>(A.flt.f[tid]);
+  if (!sched_layout)  // scheduled calls read the A-column from its table
+    for (int i = tid; i < g.n_theta * (g.bins + 1); i += nthreads) sH[i] = gH[i];
+  for (int v = tid; v < g.n_theta; v += nthreads) {
+    if (kF32)
+      sbx[v] = A.tab.bx[v];
+    else
+      sbxd[v] = A.tab.bxd[v];
+    sgw[v] = ggw[v];
   }
+  if (tid < kMaxTRows) shv[tid] = ghv[y * kMaxTRows + tid];
   if (tid < 4) ctl[tid] = 0u;
   __syncthreads();  // constants and tables visible before any path uses them
 
@@ -1257,10 +944,6 @@ __device__ __forceinline__ bool run_slice(const SweepArgs& A, int y, unsigned ch
 #pragma unroll
   for (int s2 = 0; s2 < kStatSlots; ++s2) acc.v[s2] = 0ull;
   unsigned skipped = 0;
-  TabCtx<G, VPL, BF> tc;
-  if constexpr (TAB)
-    tab_ctx<G, VPL, STAGE, BF>(tc, A, y, es, rs, c.bw, c.bs, c.bs_rs, ghv[y * kMaxTRows], cache,
-                               sched_layout, coherent, lane);
   // Level schedule: the call's lines level by level, one CTA barrier per level; neighbours are
   // read from the volume (the slice's own plane is written only by this CTA, the planes y+-1
   // belong to the other colour and do not change during the launch), the zero-skipping test
@@ -1312,10 +995,7 @@ __device__ __forceinline__ bool run_slice(const SweepArgs& A, int y, unsigned ch
               x = l - z * g.n_x;
             }
           }
-          if constexpr (TAB)
-            table_step<G, VPL, STAGE, BF, true>(A, tc, z, x, act, lane, zs_on, acc);
-          else
-            group_step<Real, NB, G, VPL, BF, false, true>(c, z, x, y, act, lane, acc);
+          group_step<Real, NB, G, VPL, BF, false, true>(c, z, x, y, act, lane, acc);
         }
         __syncthreads();
       }
@@ -1324,7 +1004,7 @@ __device__ __forceinline__ bool run_slice(const SweepArgs& A, int y, unsigned ch
   for (int rr = 0; !scheduled && rr < g.n_z; ++rr) {
     const int z = A.row_order[rr];
     __syncthreads();
-    if constexpr (!TAB) compute_row_base<Real>(A.tab, g.n_theta, z, rb, tid, nthreads);
+    compute_row_base<Real>(A.tab, g.n_theta, z, rb, tid, nthreads);
     // neighbour rows (y+dy, z+dz), dy, dz in {-1,0,1} (rows outside the volume read as 0),
     // loaded column by column: each thread also records whether its column holds a value > 0
     // (bit 2 of lv), from which the zero-skipping test of every voxel follows
@@ -1474,15 +1154,7 @@ __device__ __forceinline__ bool run_slice(const SweepArgs& A, int y, unsigned ch
       for (int b0 = 0; b0 < n; b0 += n_groups) {
         const int i = b0 + group;
         const bool act = i < n;
-        if constexpr (TAB) {
-          if (project)
-            table_project<G, VPL, STAGE, BF>(A, tc, z, act ? flat[b + i] : 0, act, lane);
-          else
-            table_step<G, VPL, STAGE, BF, false>(A, tc, z, act ? flat[b + i] : 0, act, lane, zs_on,
-                                                 acc);
-        } else {
-          group_step<Real, NB, G, VPL, BF, false>(c, z, act ? flat[b + i] : 0, y, act, lane, acc);
-        }
+        group_step<Real, NB, G, VPL, BF, false>(c, z, act ? flat[b + i] : 0, y, act, lane, acc);
       }
       __syncthreads();
     }
@@ -1530,7 +1202,7 @@ __device__ __forceinline__ void init_slice_barrier(unsigned char* smem) {
 }
 
 // One launch = the slices of one y-colour of one reconstruction, one CTA per slice.
-template <typename Real, int NB, int G, int VPL, bool STAGE, bool BF, bool TAB>
+template <typename Real, int NB, int G, int VPL, bool STAGE, bool BF>
 __global__ void __launch_bounds__(kWarps * 32, 1) sweep_kernel(const __grid_constant__ SweepArgs A) {
   extern __shared__ __align__(128) unsigned char smem[];
   // slab launches (y_end > 0) start at y_first; whole-volume launches at the colour
@@ -1538,31 +1210,32 @@ __global__ void __launch_bounds__(kWarps * 32, 1) sweep_kernel(const __grid_cons
   if (y >= (A.y_end > 0 ? A.y_end : A.g.n_y)) return;
   init_slice_barrier(smem);
   uint32_t phase = 0;
-  run_slice<Real, NB, G, VPL, STAGE, BF, TAB>(
+  run_slice<Real, NB, G, VPL, STAGE, BF>(
       A, y, smem, phase, false,
       A.stats != nullptr ? A.stats + static_cast<size_t>(blockIdx.x) * kStatSlots : nullptr);
 }
 
 // One slice of a batched series with its staging.
-template <int NB, int G, int VPL, bool BF, bool TAB>
+template <int NB, int G, int VPL, bool BF>
 __device__ __forceinline__ void batch_slice(const SweepArgs& sA, int y, unsigned char* smem,
                                             uint32_t& phase, double* stat_out) {
   if (sA.smem_rows)
-    run_slice<float, NB, G, VPL, true, BF, TAB>(sA, y, smem, phase, true, stat_out);
+    run_slice<float, NB, G, VPL, true, BF>(sA, y, smem, phase, true, stat_out);
   else
-    run_slice<float, NB, G, VPL, false, BF, TAB>(sA, y, smem, phase, true, stat_out);
+    run_slice<float, NB, G, VPL, false, BF>(sA, y, smem, phase, true, stat_out);
 }
 
 // Many reconstructions of uneven size in one persistent launch per sweep (FP32).  CTAs pull
 // (series, slice) items from a queue: first every colour-0 slice, then every colour-1 slice.
 // A colour-1 slice needs the colour-0 neighbours y+-1 of its own series, so it waits (with a
 // time bound) until all colour-0 slices of that series are done; those were taken from the
-// queue earlier by running CTAs, so the wait always ends.  Launched cooperatively so every CTA
-// is resident.  One launch covers the series of one voxel-group shape; it may use 256 threads
-// per CTA (two CTAs per SM under the 128-register cap) or 512.  Bright-field and HAADF series,
-// and table-driven series and others, run in separate launches.
-template <int NB, int G, int VPL, bool BF, bool TAB>
-__global__ void __launch_bounds__(kWarps * 32, 1) batch_sweep_kernel(BatchArgs B) {
+// queue earlier by running CTAs, so the wait always ends whatever CTAs are resident, and the
+// launches of a sweep run side by side on streams of their own: as one drains, the next one's
+// CTAs take its SMs.  One launch covers the series of one voxel-group shape; it may use 256 threads
+// per CTA (two CTAs per SM under the 128-register cap) or 512.  Bright-field and HAADF series
+// run in separate launches.
+template <typename F>
+__device__ __forceinline__ void batch_items(const BatchArgs& B, F slice) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ SweepArgs sA;
   __shared__ int s_item;
@@ -1601,13 +1274,20 @@ __global__ void __launch_bounds__(kWarps * 32, 1) batch_sweep_kernel(BatchArgs B
     if (!s_wait_ok) continue;
     const int n0 = (sA.g.n_y + 1) / 2;
     const int slot = (y & 1) ? n0 + (y >> 1) : (y >> 1);
-    double* stat_out = sA.stats + static_cast<size_t>(slot) * kStatSlots;
-    batch_slice<NB, G, VPL, BF, TAB>(sA, y, smem, phase, stat_out);
+    slice(sA, y, smem, phase, sA.stats + static_cast<size_t>(slot) * kStatSlots);
     if (threadIdx.x == 0 && !(y & 1)) {
       __threadfence();
       atomicAdd(B.done + s, 1);
     }
   }
+}
+
+template <int NB, int G, int VPL, bool BF>
+__global__ void __launch_bounds__(kWarps * 32, 1) batch_sweep_kernel(BatchArgs B) {
+  batch_items(B, [](const SweepArgs& sA, int y, unsigned char* smem, uint32_t& phase,
+                    double* stat_out) {
+    batch_slice<NB, G, VPL, BF>(sA, y, smem, phase, stat_out);
+  });
 }
 
 // The reference's visit order: voxel lines one after another in list order, y ascending
@@ -1761,27 +1441,32 @@ inline int launch_acol_t(const DevGeom& g, const DevTables& tab, int nb, float4*
   return ok_or(cudaGetLastError());
 }
 
-template <typename Real, int NB, int G, int VPL, bool STAGE, bool BF, bool TAB = false>
-int launch_sweep_t(const SweepArgs& a, size_t smem, cudaStream_t s) {
-  auto k = sweep_kernel<Real, NB, G, VPL, STAGE, BF, TAB>;
+// Launch of a kernel with one CTA per slice
+template <auto k>
+int launch_slices(const SweepArgs& a, size_t smem, int threads, cudaStream_t s) {
   static const int lim = dyn_smem_limit(k);
   if (smem > static_cast<size_t>(lim)) return -3;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   if (e != cudaSuccess) return -3;
   // shared-memory carveout just large enough for this launch: the rest of the SM's unified
   // L1/shared storage caches the gathered weights and neighbour rows
-  static int per_sm = 0;
-  if (per_sm == 0) {
-    int dev = 0;
+  static const int per_sm = [] {
+    int dev = 0, v = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-  }
+    cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+    return v;
+  }();
   if (per_sm > 0) {
     const int pct = static_cast<int>(std::min<size_t>(100, (100 * (smem + 4096) + per_sm - 1) / per_sm));
     cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
   }
-  k<<<a.n_slices, kWarps * 32, smem, s>>>(a);
+  k<<<a.n_slices, threads, smem, s>>>(a);
   return ok_or(cudaGetLastError());
+}
+
+template <typename Real, int NB, int G, int VPL, bool STAGE, bool BF>
+int launch_sweep_t(const SweepArgs& a, size_t smem, cudaStream_t s) {
+  return launch_slices<sweep_kernel<Real, NB, G, VPL, STAGE, BF>>(a, smem, kWarps * 32, s);
 }
 template <typename Real, int NB, int G, int VPL, bool STAGE>
 int launch_sweep_m(const SweepArgs& a, size_t smem, cudaStream_t s) {
@@ -1789,9 +1474,8 @@ int launch_sweep_m(const SweepArgs& a, size_t smem, cudaStream_t s) {
               : launch_sweep_t<Real, NB, G, VPL, STAGE, false>(a, smem, s);
 }
 
-template <int NB, int G, int VPL, bool BF, bool TAB>
-int launch_batch_t(const BatchArgs& b, size_t smem, int grid, int threads, cudaStream_t s) {
-  auto k = batch_sweep_kernel<NB, G, VPL, BF, TAB>;
+template <auto k>
+int launch_batch_kernel(const BatchArgs& b, size_t smem, int grid, int threads, cudaStream_t s) {
   static const int lim = dyn_smem_limit(k);
   if (smem > static_cast<size_t>(lim)) return -3;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
@@ -1805,11 +1489,13 @@ int launch_batch_t(const BatchArgs& b, size_t smem, int grid, int threads, cudaS
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (grid <= 0 || grid > per_sm * sms) grid = per_sm * sms;
-  BatchArgs arg = b;
-  void* params[] = {&arg};
-  e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k), dim3(grid), dim3(threads), params,
-                                  smem, s);
-  return ok_or(e);
+  k<<<std::min(grid, b.n_items), threads, smem, s>>>(b);
+  return ok_or(cudaGetLastError());
+}
+
+template <int NB, int G, int VPL, bool BF>
+int launch_batch_t(const BatchArgs& b, size_t smem, int grid, int threads, cudaStream_t s) {
+  return launch_batch_kernel<batch_sweep_kernel<NB, G, VPL, BF>>(b, smem, grid, threads, s);
 }
 
 template <typename Real, int NB, int VPL>
@@ -1833,14 +1519,6 @@ template <bool STAGE, bool BF>
 int launch_sweep_f32_pick(const SweepArgs& a, int nb, size_t smem, cudaStream_t s) {
   // explicit shape (1..4) when it covers the views, else the default for the view count
   const int shape = resolved_shape(a.shape, a.g.n_theta);
-  if (table_driven(a, nb)) {
-    if (shape == 1) return launch_sweep_t<float, 3, 16, 4, STAGE, BF, true>(a, smem, s);
-    if (shape == 2) return launch_sweep_t<float, 3, 32, 2, STAGE, BF, true>(a, smem, s);
-    if (shape == 3) return launch_sweep_t<float, 3, 32, 3, STAGE, BF, true>(a, smem, s);
-    if (shape == 4) return launch_sweep_t<float, 3, 32, 5, STAGE, BF, true>(a, smem, s);
-    if constexpr (!STAGE) return launch_sweep_t<float, 3, 32, 8, STAGE, BF, true>(a, smem, s);
-    return -7;
-  }
   if constexpr (!STAGE) {  // more than 160 views: 32 lanes x 8 views, slices in HBM
     if (shape == 5) {
       if (nb == 3) return launch_sweep_t<float, 3, 32, 8, STAGE, BF>(a, smem, s);
@@ -1867,23 +1545,22 @@ int launch_sweep_f32_pick(const SweepArgs& a, int nb, size_t smem, cudaStream_t 
   return -7;
 }
 
-// The voxel-group shape of every series in the launch (1 = 16x4, 2 = 32x2, 3 = 32x3, 4 = 32x5),
-// whether they are bright field and whether they are table-driven (batch_group)
-template <int NB, bool BF, bool TAB>
+// The voxel-group shape of every series in the launch (1 = 16x4, 2 = 32x2, 3 = 32x3, 4 = 32x5)
+// and whether they are bright field (batch_group)
+template <int NB, bool BF>
 int launch_batch_shape(const BatchArgs& b, int shape, int threads, size_t smem, int grid,
                        cudaStream_t s) {
-  if (shape == 1) return launch_batch_t<NB, 16, 4, BF, TAB>(b, smem, grid, threads, s);
-  if (shape == 2) return launch_batch_t<NB, 32, 2, BF, TAB>(b, smem, grid, threads, s);
-  if (shape == 3) return launch_batch_t<NB, 32, 3, BF, TAB>(b, smem, grid, threads, s);
-  return launch_batch_t<NB, 32, 5, BF, TAB>(b, smem, grid, threads, s);
+  if (shape == 1) return launch_batch_t<NB, 16, 4, BF>(b, smem, grid, threads, s);
+  if (shape == 2) return launch_batch_t<NB, 32, 2, BF>(b, smem, grid, threads, s);
+  if (shape == 3) return launch_batch_t<NB, 32, 3, BF>(b, smem, grid, threads, s);
+  return launch_batch_t<NB, 32, 5, BF>(b, smem, grid, threads, s);
 }
-template <int NB, bool TAB>
+template <int NB>
 int launch_batch_pick(const BatchArgs& b, int group, int threads, size_t smem, int grid,
                       cudaStream_t s) {
   return batch_group_bf(group)
-             ? launch_batch_shape<NB, true, TAB>(b, batch_group_shape(group), threads, smem, grid, s)
-             : launch_batch_shape<NB, false, TAB>(b, batch_group_shape(group), threads, smem, grid,
-                                                  s);
+             ? launch_batch_shape<NB, true>(b, batch_group_shape(group), threads, smem, grid, s)
+             : launch_batch_shape<NB, false>(b, batch_group_shape(group), threads, smem, grid, s);
 }
 
 }  // namespace sweep

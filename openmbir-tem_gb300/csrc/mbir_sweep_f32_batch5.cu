@@ -5,7 +5,7 @@ namespace mbir {
 
 int launch_batch_sweep_nb5(const BatchArgs& b, int group, int threads, size_t smem, int grid,
                             void* stream) {
-  return sweep::launch_batch_pick<5, false>(b, group, threads, smem, grid,
+  return sweep::launch_batch_pick<5>(b, group, threads, smem, grid,
                                      static_cast<cudaStream_t>(stream));
 }
 
