@@ -19,7 +19,10 @@
 // arithmetic.  Elementwise passes are the same in both modes.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "mbir_internal.h"
+#include "mbir_wide.cuh"
 
 namespace mbir {
 
@@ -96,6 +99,21 @@ __device__ __forceinline__ void offset_term(double ev, double w, bool sel, doubl
   }
 }
 
+// one variance-sum term (BFForwardModel.cpp:470-480); w already multiplied by alpha_view
+__device__ __forceinline__ void variance_term(double ev, double w, double a, bool sel,
+                                              double& s1, double& s2) {
+  if (sel)
+    s1 += (ev * ev * w);
+  else
+    s2 += fabs(ev) * sqrt(a * w);
+}
+
+// one data-term entry of forwardCost (BFForwardModel.cpp:822-830)
+__device__ __forceinline__ double cost_term(double ev, double w, bool sel, double T, double dl) {
+  if (sel) return (ev * ev * w);
+  return (2 * T * dl * fabs(ev) * sqrt(w) + T * T * (1 - 2 * dl));
+}
+
 template <typename Real>
 __global__ void offset_sums_kernel(const Real* __restrict__ e, const Real* __restrict__ w,
                                    const uint8_t* __restrict__ sel, double T, double dl,
@@ -126,6 +144,222 @@ __global__ void chunk_final_kernel(const double* __restrict__ partial, double* _
   double s = 0.0;
   for (int c = 0; c < n_chunk; ++c) s += partial[(static_cast<size_t>(v) * n_chunk + c) * K + k];
   out[i] = s;
+}
+
+// ---- FP32 engine: the same passes with FP64-accurate sums and roundings on the FP32 units
+// (mbir_wide.cuh).  With their arithmetic in FP64 the five passes of an offset and a variance
+// update took 0.5 ms of 8 M entries (73 MB, in L2 mostly: about 60 us); the two updates now make
+// four: offset sums, offset step and selector, variance sums, new weights and selector.
+
+// four selector bytes (rows of a multiple of 16)
+__device__ __forceinline__ void sel4(const uint8_t* sel, size_t i, bool (&on)[4]) {
+  const uchar4 s = *reinterpret_cast<const uchar4*>(sel + i);
+  on[0] = s.x == 1;
+  on[1] = s.y == 1;
+  on[2] = s.z == 1;
+  on[3] = s.w == 1;
+}
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+  const float4 q = *reinterpret_cast<const float4*>(p);
+  v[0] = q.x;
+  v[1] = q.y;
+  v[2] = q.z;
+  v[3] = q.w;
+}
+
+// Per view and chunk of rows two sums of selected entries (WideSum) and rejected ones (FP64).
+// term(e, w, a) is the selected entry's contribution, kind by kind.
+enum SumKind { kOffsetSums = 0, kVarianceSums = 1, kCostSums = 2 };
+
+// (float)((double)w * a)
+__device__ __forceinline__ float weight_times(float w, double a, wide::F2 af) {
+  const wide::F2 p = wide::mul(af, w);
+  float r;
+  if (!wide::rounds_to(p, 1.2e-13f * fabsf(p.hi), r))
+    r = static_cast<float>(static_cast<double>(w) * a);
+  return r;
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(256)
+    sums_f32_kernel(const float* __restrict__ e, float* __restrict__ w,
+                    const uint8_t* __restrict__ sel, const double* __restrict__ alpha, int store,
+                    double T, double dl, int n_theta, int n_rp, int n_sp, int n_r, int n_t,
+                    int n_chunk, double* __restrict__ partial) {
+  const int v = blockIdx.x, ch = blockIdx.y;
+  const int t0 = static_cast<int>(static_cast<long long>(ch) * n_t / n_chunk);
+  const int t1 = static_cast<int>(static_cast<long long>(ch + 1) * n_t / n_chunk);
+  const double a = KIND == kVarianceSums ? alpha[v] : 1.0;
+  const wide::F2 af = wide::split(a);
+  double acc[2] = {0.0, 0.0};
+  wide::WideSum sum[2];
+  bool any = false;
+  wide::for_view_rows(
+      v, t0, t1, n_theta, n_rp,
+      [&](size_t row, int r) {
+        const size_t base = row * n_rp;
+        float ev[4], wv[4];
+        bool on[4];
+        load4(e + base + r, ev);
+        load4(w + base + r, wv);
+        sel4(sel, row * n_sp + r, on);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (r + j >= n_r) continue;
+          if constexpr (KIND == kVarianceSums) wv[j] = weight_times(wv[j], a, af);
+          if (on[j]) {
+            any = true;
+            if constexpr (KIND == kOffsetSums) {
+              sum[0].add(wide::two_prod(ev[j], wv[j]));
+              sum[1].add(wv[j]);
+            } else {
+              sum[0].add(wide::mul(wide::two_prod(ev[j], ev[j]), wv[j]));
+            }
+          } else if constexpr (KIND == kOffsetSums) {
+            offset_term(ev[j], wv[j], false, T, dl, acc[0], acc[1]);
+          } else if constexpr (KIND == kVarianceSums) {
+            variance_term(ev[j], wv[j], a, false, acc[0], acc[1]);
+          } else {
+            acc[0] += cost_term(ev[j], wv[j], false, T, dl);
+          }
+        }
+        if constexpr (KIND == kVarianceSums) {
+          if (store) *reinterpret_cast<float4*>(w + base + r) = make_float4(wv[0], wv[1], wv[2], wv[3]);
+        }
+      },
+      [&](auto again) {
+        const bool sound = sum[0].sound() && (KIND != kOffsetSums || sum[1].sound());
+        if (sound) {
+          acc[0] += sum[0].value();
+          if constexpr (KIND == kOffsetSums) acc[1] += sum[1].value();
+        } else if (any) {
+          again([&](size_t row, int r) {
+            const size_t base = row * n_rp;
+            for (int j = 0; j < 4 && r + j < n_r; ++j) {
+              if (sel[row * n_sp + r + j] != 1) continue;
+              const double ed = e[base + r + j];
+              double wd = w[base + r + j];
+              if constexpr (KIND == kOffsetSums) {
+                acc[0] += ed * wd;
+                acc[1] += wd;
+              } else {
+                if constexpr (KIND == kVarianceSums)
+                  if (!store) wd = static_cast<float>(wd * a);
+                acc[0] += ed * ed * wd;
+              }
+            }
+          });
+        }
+        sum[0] = wide::WideSum();
+        sum[1] = wide::WideSum();
+        any = false;
+      });
+  const double s = wide::block_sums<2>(acc);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp < 2 && lane == 0) partial[(static_cast<size_t>(v) * n_chunk + ch) * 2 + warp] = s;
+}
+
+// e -= step of the view, then the selector (offset_apply_kernel and selector_kernel)
+__global__ void __launch_bounds__(256)
+    offset_step_f32_kernel(float* __restrict__ e, const float* __restrict__ w,
+                           uint8_t* __restrict__ sel, const double* __restrict__ step, double T,
+                           int n_theta, int n_rp, int n_sp, int n_r, int n_t, int n_chunk) {
+  const int v = blockIdx.x, ch = blockIdx.y;
+  const int t0 = static_cast<int>(static_cast<long long>(ch) * n_t / n_chunk);
+  const int t1 = static_cast<int>(static_cast<long long>(ch + 1) * n_t / n_chunk);
+  const double st = step[v], t2 = T * T;
+  const wide::F2 sf = wide::neg(wide::split(st));
+  const float t2f = static_cast<float>(t2);
+  wide::for_view_rows(
+      v, t0, t1, n_theta, n_rp,
+      [&](size_t row, int r) {
+        const size_t base = row * n_rp;
+        float ev[4], wv[4];
+        load4(e + base + r, ev);
+        load4(w + base + r, wv);
+        const size_t si = row * n_sp + r;
+        uint8_t on[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          on[j] = 0;
+          if (r + j >= n_r) continue;
+          const wide::F2 d = wide::add(wide::two_sum(ev[j], sf.hi), wide::F2{sf.lo, 0.f});
+          float o;
+          if (!wide::rounds_to(d, 1.2e-13f * (fabsf(ev[j]) + fabsf(sf.hi)), o))
+            o = static_cast<float>(static_cast<double>(ev[j]) - st);
+          ev[j] = o;
+          on[j] = wide::below(o, wv[j], t2, t2f) ? 1 : 0;
+        }
+        *reinterpret_cast<float4*>(e + base + r) = make_float4(ev[0], ev[1], ev[2], ev[3]);
+        if (r + 3 < n_r) {
+          *reinterpret_cast<uchar4*>(sel + si) = make_uchar4(on[0], on[1], on[2], on[3]);
+        } else {
+          for (int j = 0; j < 4 && r + j < n_r; ++j) sel[si + j] = on[j];
+        }
+      },
+      [](auto) {});
+}
+
+// w = (float)((float)(w alpha_view) / upd), then the selector (variance_sums_kernel's scaling,
+// scale_weights_kernel and selector_kernel)
+__global__ void __launch_bounds__(256)
+    new_weights_f32_kernel(const float* __restrict__ e, float* __restrict__ w,
+                           uint8_t* __restrict__ sel, const double* __restrict__ alpha, double upd,
+                           double T, int n_theta, int n_rp, int n_sp, int n_r, int n_t,
+                           int n_chunk) {
+  const int v = blockIdx.x, ch = blockIdx.y;
+  const int t0 = static_cast<int>(static_cast<long long>(ch) * n_t / n_chunk);
+  const int t1 = static_cast<int>(static_cast<long long>(ch + 1) * n_t / n_chunk);
+  const double a = alpha[v], t2 = T * T;
+  const wide::F2 af = wide::split(a), inv = wide::split(1.0 / upd);
+  const float t2f = static_cast<float>(t2);
+  wide::for_view_rows(
+      v, t0, t1, n_theta, n_rp,
+      [&](size_t row, int r) {
+        const size_t base = row * n_rp;
+        float ev[4], wv[4];
+        load4(e + base + r, ev);
+        load4(w + base + r, wv);
+        const size_t si = row * n_sp + r;
+        uint8_t on[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          on[j] = 0;
+          if (r + j >= n_r) continue;
+          const float w1 = weight_times(wv[j], a, af);
+          const wide::F2 q = wide::mul(inv, w1);
+          if (!wide::rounds_to(q, 1.2e-13f * fabsf(q.hi), wv[j]))
+            wv[j] = static_cast<float>(static_cast<double>(w1) / upd);
+          on[j] = wide::below(ev[j], wv[j], t2, t2f) ? 1 : 0;
+        }
+        *reinterpret_cast<float4*>(w + base + r) = make_float4(wv[0], wv[1], wv[2], wv[3]);
+        if (r + 3 < n_r) {
+          *reinterpret_cast<uchar4*>(sel + si) = make_uchar4(on[0], on[1], on[2], on[3]);
+        } else {
+          for (int j = 0; j < 4 && r + j < n_r; ++j) sel[si + j] = on[j];
+        }
+      },
+      [](auto) {});
+}
+
+// Column sums of partial [n][K] (256 threads)
+template <int K>
+__global__ void __launch_bounds__(256)
+    partials_final_kernel(const double* __restrict__ partial, double* __restrict__ out, int n) {
+  double acc[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) acc[k] = 0.0;
+  for (int i = threadIdx.x; i < n; i += 256)
+#pragma unroll
+    for (int k = 0; k < K; ++k) acc[k] += partial[static_cast<size_t>(i) * K + k];
+  const double s = wide::block_sums<K>(acc);
+  if ((threadIdx.x & 31) == 0 && (threadIdx.x >> 5) < K) out[threadIdx.x >> 5] = s;
+}
+
+// Row chunks per view: about 2000 blocks, their partials within the 4096 doubles of the engine's
+// bright-field scratch
+inline int view_chunks(const BfSino& b) {
+  return std::max(1, std::min(b.n_t, 2000 / std::max(1, b.n_theta)));
 }
 
 // reference order: one thread per view, r then t
@@ -174,15 +408,6 @@ __global__ void selector_kernel(const Real* __restrict__ e, const Real* __restri
     const double ev = e[k];
     sel[i] = (ev * ev * static_cast<double>(w[k]) < T * T) ? 1 : 0;
   }
-}
-
-// one variance-sum term (BFForwardModel.cpp:470-480); w already multiplied by alpha_view
-__device__ __forceinline__ void variance_term(double ev, double w, double a, bool sel,
-                                              double& s1, double& s2) {
-  if (sel)
-    s1 += (ev * ev * w);
-  else
-    s2 += fabs(ev) * sqrt(a * w);
 }
 
 template <typename Real>
@@ -254,12 +479,6 @@ __global__ void scale_weights_kernel(Real* __restrict__ w, double alpha, int n_t
     if (r >= n_r) continue;
     w[i] = static_cast<Real>(static_cast<double>(w[i]) / alpha);
   }
-}
-
-// one data-term entry of forwardCost (BFForwardModel.cpp:822-830)
-__device__ __forceinline__ double cost_term(double ev, double w, bool sel, double T, double dl) {
-  if (sel) return (ev * ev * w);
-  return (2 * T * dl * fabs(ev) * sqrt(w) + T * T * (1 - 2 * dl));
 }
 
 template <typename Real>
@@ -409,9 +628,9 @@ int launch_bf_offset_sums(const BfSino& b, int exact, double T, double dl, doubl
                                                     b.n_theta, b.n_rp, b.n_sp, b.n_r, b.n_t, n_chunk,
                                                     partial);
   else
-    offset_sums_kernel<float><<<grid, 256, 0, s>>>(RP<float>(b.e), RP<float>(b.w), b.sel, T, dl,
-                                                   b.n_theta, b.n_rp, b.n_sp, b.n_r, b.n_t, n_chunk,
-                                                   partial);
+    sums_f32_kernel<kOffsetSums><<<grid, 256, 0, s>>>(RP<float>(b.e), RP<float>(b.w), b.sel, nullptr,
+                                                      0, T, dl, b.n_theta, b.n_rp, b.n_sp, b.n_r,
+                                                      b.n_t, n_chunk, partial);
   const int n = b.n_theta * 2;
   chunk_final_kernel<<<(n + 127) / 128, 128, 0, s>>>(partial, out, b.n_theta, n_chunk, 2);
   return ok_or(cudaGetLastError());
@@ -442,8 +661,8 @@ int launch_bf_selector(const BfSino& b, double T, void* stream) {
   return ok_or(cudaGetLastError());
 }
 
-int launch_bf_variance_sums(const BfSino& b, int exact, const double* alpha, double* partial,
-                            double* out, void* stream) {
+int launch_bf_variance_sums(const BfSino& b, int exact, const double* alpha, bool scale,
+                            double* partial, double* out, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (exact) {
     if (b.fp64)
@@ -455,15 +674,38 @@ int launch_bf_variance_sums(const BfSino& b, int exact, const double* alpha, dou
                                                        b.n_theta, b.n_rp, b.n_sp, b.n_r, b.n_t, out);
     return ok_or(cudaGetLastError());
   }
-  if (b.fp64)
+  if (b.fp64) {
     variance_sums_kernel<double><<<kRedBlocks, 256, 0, s>>>(RP<double>(b.e), RP<double>(b.w), b.sel,
                                                             alpha, b.n_theta, b.n_rp, b.n_sp, b.n_r,
                                                             b.n_t, partial);
-  else
-    variance_sums_kernel<float><<<kRedBlocks, 256, 0, s>>>(RP<float>(b.e), RP<float>(b.w), b.sel,
-                                                           alpha, b.n_theta, b.n_rp, b.n_sp, b.n_r,
-                                                           b.n_t, partial);
-  blocks_final_kernel<<<1, 32, 0, s>>>(partial, out, kRedBlocks, 2);
+    blocks_final_kernel<<<1, 32, 0, s>>>(partial, out, kRedBlocks, 2);
+    return ok_or(cudaGetLastError());
+  }
+  const int chunks = view_chunks(b);
+  sums_f32_kernel<kVarianceSums><<<dim3(b.n_theta, chunks), 256, 0, s>>>(
+      RP<float>(b.e), RP<float>(b.w), b.sel, alpha, scale ? 1 : 0, 0.0, 0.0, b.n_theta, b.n_rp,
+      b.n_sp, b.n_r, b.n_t, chunks, partial);
+  partials_final_kernel<2><<<1, 256, 0, s>>>(partial, out, b.n_theta * chunks);
+  return ok_or(cudaGetLastError());
+}
+
+// FP32 engine: the offset step and the selector that follows it, in one pass
+int launch_bf_offset_step(const BfSino& b, const double* step, double T, void* stream) {
+  const int chunks = view_chunks(b);
+  offset_step_f32_kernel<<<dim3(b.n_theta, chunks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      RP<float>(b.e), RP<float>(b.w), b.sel, step, T, b.n_theta, b.n_rp, b.n_sp, b.n_r, b.n_t,
+      chunks);
+  return ok_or(cudaGetLastError());
+}
+
+// FP32 engine: the weights of the new common variance (after variance sums that did not scale
+// them) and the selector that follows, in one pass
+int launch_bf_new_weights(const BfSino& b, const double* alpha, double upd, double T,
+                          void* stream) {
+  const int chunks = view_chunks(b);
+  new_weights_f32_kernel<<<dim3(b.n_theta, chunks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      RP<float>(b.e), RP<float>(b.w), b.sel, alpha, upd, T, b.n_theta, b.n_rp, b.n_sp, b.n_r, b.n_t,
+      chunks);
   return ok_or(cudaGetLastError());
 }
 
@@ -491,15 +733,18 @@ int launch_bf_cost_sums(const BfSino& b, int exact, double T, double dl, double*
                                                    b.n_theta, b.n_rp, b.n_sp, b.n_r, b.n_t, out);
     return ok_or(cudaGetLastError());
   }
-  if (b.fp64)
+  if (b.fp64) {
     cost_sums_kernel<double><<<kRedBlocks, 256, 0, s>>>(RP<double>(b.e), RP<double>(b.w), b.sel, T,
                                                         dl, b.n_theta, b.n_rp, b.n_sp, b.n_r, b.n_t,
                                                         partial);
-  else
-    cost_sums_kernel<float><<<kRedBlocks, 256, 0, s>>>(RP<float>(b.e), RP<float>(b.w), b.sel, T, dl,
-                                                       b.n_theta, b.n_rp, b.n_sp, b.n_r, b.n_t,
-                                                       partial);
-  blocks_final_kernel<<<1, 32, 0, s>>>(partial, out, kRedBlocks, 1);
+    blocks_final_kernel<<<1, 32, 0, s>>>(partial, out, kRedBlocks, 1);
+    return ok_or(cudaGetLastError());
+  }
+  const int chunks = view_chunks(b);
+  sums_f32_kernel<kCostSums><<<dim3(b.n_theta, chunks), 256, 0, s>>>(
+      RP<float>(b.e), RP<float>(b.w), b.sel, nullptr, 0, T, dl, b.n_theta, b.n_rp, b.n_sp, b.n_r,
+      b.n_t, chunks, partial);
+  partials_final_kernel<2><<<1, 256, 0, s>>>(partial, out, b.n_theta * chunks);
   return ok_or(cudaGetLastError());
 }
 

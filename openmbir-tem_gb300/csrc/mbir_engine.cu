@@ -119,11 +119,9 @@ void Engine::release() {
   dfree(d_lines_);
   dfree(d_stats_);
   dfree(d_stat4_);
-  dfree(d_mu_);
-  dfree(d_gain_);
+  d_mu_ = d_gain_ = d_wv_ = nullptr;  // parts of d_gw_
   dfree(d_mu2_);
   dfree(d_gain2_);
-  dfree(d_wv_);
   dfree(d_partial_);
   dfree(d_vsum_);
   dfree(d_err_);
@@ -652,7 +650,16 @@ int Engine::alloc_device() {
   rc |= dmalloc(&d_bxd_, g.n_theta);
   rc |= dmalloc(&d_u0_, g.n_theta);
   rc |= dmalloc(&d_bz_, g.n_theta);
-  rc |= dmalloc_bytes(&d_gw_, static_cast<size_t>(g.n_theta) * 2 * rb_);
+  {
+    const size_t gw = (static_cast<size_t>(g.n_theta) * 2 * rb_ + 15) / 16 * 16;
+    views_bytes_ = gw + 3 * sizeof(double) * static_cast<size_t>(g.n_theta);
+    rc |= dmalloc_bytes(&d_gw_, views_bytes_);
+    if (!rc) {
+      d_mu_ = reinterpret_cast<double*>(static_cast<char*>(d_gw_) + gw);
+      d_gain_ = d_mu_ + g.n_theta;
+      d_wv_ = d_gain_ + g.n_theta;
+    }
+  }
   rc |= dmalloc(&d_tfirst_, g.n_y);
   rc |= dmalloc(&d_tcount_, g.n_y);
   rc |= dmalloc_bytes(&d_hval_, static_cast<size_t>(g.n_y) * kMaxTRows * rb_);
@@ -719,20 +726,20 @@ int Engine::alloc_device() {
 int Engine::upload_views() {
   const int nt = g_.n_theta;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  std::vector<float2> gw(nt);
-  std::vector<double2> gwd(nt);
+  std::vector<unsigned char> host(views_bytes_);
+  const unsigned char* base = static_cast<const unsigned char*>(d_gw_);
+  auto at = [&](const void* d) { return host.data() + (static_cast<const unsigned char*>(d) - base); };
   for (int v = 0; v < nt; v++) {
-    gw[v] = make_float2(static_cast<float>(I_[v]), static_cast<float>(w_[v]));
-    gwd[v] = make_double2(I_[v], w_[v]);
+    if (fp64_)
+      reinterpret_cast<double2*>(host.data())[v] = make_double2(I_[v], w_[v]);
+    else
+      reinterpret_cast<float2*>(host.data())[v] =
+          make_float2(static_cast<float>(I_[v]), static_cast<float>(w_[v]));
   }
-  if (fp64_)
-    cudaMemcpyAsync(d_gw_, gwd.data(), sizeof(double2) * nt, cudaMemcpyHostToDevice, s);
-  else
-    cudaMemcpyAsync(d_gw_, gw.data(), sizeof(float2) * nt, cudaMemcpyHostToDevice, s);
-  cudaStreamSynchronize(s);  // host vectors go out of scope
-  cudaMemcpyAsync(d_mu_, mu_.data(), sizeof(double) * nt, cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(d_gain_, I_.data(), sizeof(double) * nt, cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(d_wv_, w_.data(), sizeof(double) * nt, cudaMemcpyHostToDevice, s);
+  std::copy(mu_.begin(), mu_.begin() + nt, reinterpret_cast<double*>(at(d_mu_)));
+  std::copy(I_.begin(), I_.begin() + nt, reinterpret_cast<double*>(at(d_gain_)));
+  std::copy(w_.begin(), w_.begin() + nt, reinterpret_cast<double*>(at(d_wv_)));
+  cudaMemcpyAsync(d_gw_, host.data(), views_bytes_, cudaMemcpyHostToDevice, s);
   return cudaStreamSynchronize(s) == cudaSuccess ? 0 : cuda_check(MBIR_EDEVICE, "upload views");
 }
 

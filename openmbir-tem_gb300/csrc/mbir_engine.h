@@ -305,6 +305,7 @@ class Engine {
   double* d_mu2_ = nullptr;
   double* d_gain2_ = nullptr;
   double* d_wv_ = nullptr;
+  size_t views_bytes_ = 0;      // d_gw_, d_mu_, d_gain_ and d_wv_: one block
   double* d_partial_ = nullptr; // view sums partials
   double* d_vsum_ = nullptr;    // [n_theta*6]
   int* d_err_ = nullptr;

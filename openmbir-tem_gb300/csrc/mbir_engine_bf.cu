@@ -640,8 +640,12 @@ int Engine::bf_joint_estimation() {
     mu_[v] += step[v];
   }
   cudaMemcpyAsync(d_mu2_, step.data(), sizeof(double) * nt, cudaMemcpyHostToDevice, s);
-  if ((rc = launch_bf_offset_apply(b, d_mu2_, s))) return cuda_check(rc, "offset apply");
-  if ((rc = launch_bf_selector(b, bragg_t_, s))) return cuda_check(rc, "selector");
+  if (fp64_) {
+    if ((rc = launch_bf_offset_apply(b, d_mu2_, s))) return cuda_check(rc, "offset apply");
+    if ((rc = launch_bf_selector(b, bragg_t_, s))) return cuda_check(rc, "selector");
+  } else {
+    if ((rc = launch_bf_offset_step(b, d_mu2_, bragg_t_, s))) return cuda_check(rc, "offset step");
+  }
   if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "offset step");
   return upload_views();
 }
@@ -653,7 +657,7 @@ int Engine::bf_update_weights() {
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   const BfSino b = bf_sino();
   cudaMemcpyAsync(d_alpha_, alpha_.data(), sizeof(double) * g.n_theta, cudaMemcpyHostToDevice, s);
-  int rc = launch_bf_variance_sums(b, exact_ ? 1 : 0, d_alpha_, d_bfpart_, d_bfout_, s);
+  int rc = launch_bf_variance_sums(b, exact_ ? 1 : 0, d_alpha_, false, d_bfpart_, d_bfout_, s);
   if (rc) return cuda_check(rc, "variance sums");
   double sums[2];
   cudaMemcpyAsync(sums, d_bfout_, sizeof(sums), cudaMemcpyDeviceToHost, s);
@@ -661,8 +665,13 @@ int Engine::bf_update_weights() {
   const double upd = (sums[0] + (p_.bragg_delta * bragg_t_) * sums[1]) /
                      (g.n_theta * g.n_r * g.n_t);
   for (int v = 0; v < g.n_theta; v++) alpha_[v] = upd;
-  if ((rc = launch_bf_scale_weights(b, upd, s))) return cuda_check(rc, "weight scale");
-  if ((rc = launch_bf_selector(b, bragg_t_, s))) return cuda_check(rc, "selector");
+  if (fp64_) {
+    if ((rc = launch_bf_scale_weights(b, upd, s))) return cuda_check(rc, "weight scale");
+    if ((rc = launch_bf_selector(b, bragg_t_, s))) return cuda_check(rc, "selector");
+  } else {  // (d_alpha_ still holds the variances before this update)
+    if ((rc = launch_bf_new_weights(b, d_alpha_, upd, bragg_t_, s)))
+      return cuda_check(rc, "new weights");
+  }
   cudaMemcpyAsync(d_alpha_, alpha_.data(), sizeof(double) * g.n_theta, cudaMemcpyHostToDevice, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "variance");
   return MBIR_OK;

@@ -300,8 +300,11 @@ int launch_bf_offset_sums(const BfSino& b, int exact, double T, double dl, doubl
                           int n_chunk, double* out, void* stream);
 int launch_bf_offset_apply(const BfSino& b, const double* step, void* stream);
 int launch_bf_selector(const BfSino& b, double T, void* stream);
-int launch_bf_variance_sums(const BfSino& b, int exact, const double* alpha, double* partial,
-                            double* out, void* stream);
+// scale: the weights become w alpha (the exact mode and the FP64 engine always do that)
+int launch_bf_variance_sums(const BfSino& b, int exact, const double* alpha, bool scale,
+                            double* partial, double* out, void* stream);
+int launch_bf_offset_step(const BfSino& b, const double* step, double T, void* stream);
+int launch_bf_new_weights(const BfSino& b, const double* alpha, double upd, double T, void* stream);
 int launch_bf_scale_weights(const BfSino& b, double alpha, void* stream);
 int launch_bf_cost_sums(const BfSino& b, int exact, double T, double dl, double* partial,
                         double* out, void* stream);
@@ -375,12 +378,13 @@ int launch_vol_to_host(const void* yzx, float* zxy, int n_z, int n_x, int n_y, i
                        void* stream);
 int launch_error_from_projection(const void* y, const void* yest, void* e, const double* mu,
                                  int n_theta, int n_rp, int n_r, int n_t, int fp64, void* stream);
-// per-view FP64 sums; kind 0: joint-estimation sums (6), kind 1: sum e^2 (1)
+// per-view FP64 sums; kind 0: joint-estimation sums (6; the fifth, which the solve does not use,
+// is 0 in the FP32 engine unless all_sums), kind 1: sum e^2 (1)
 // per-view sums over detector rows [t_begin, t_end)
 int launch_view_sums_rows(int kind, const void* y, const void* e, const double* mu,
                           const double* gain, const double* wv, double* partial, double* out,
                           int n_theta, int n_rp, int n_r, int t_begin, int t_end, int n_chunk,
-                          int fp64, void* stream);
+                          int fp64, bool all_sums, void* stream);
 int launch_view_sums(int kind, const void* y, const void* e, const double* mu,
                      const double* gain, const double* wv, double* partial, double* out,
                      int n_theta, int n_rp, int n_r, int n_t, int n_chunk, int fp64,

@@ -13,105 +13,22 @@
 // HAADF_ReconstructionEngine_Extra.cpp:419-881 / HAADF_ReconstructionEngine.cpp:1147-1364.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "mbir_internal.h"
+#include "mbir_wide.cuh"
 
 namespace mbir {
 
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr uint32_t kWaitLimit = 1u << 24;  // bounded mbarrier polls before giving up
-
-template <typename Real>
-struct V2;
-template <>
-struct V2<float> {
-  using type = float2;
-};
-template <>
-struct V2<double> {
-  using type = double2;
-};
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-// ---- TMA bulk-copy helpers (cp.async.bulk + mbarrier) ------------------------------------
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
-               : "memory");
-}
-__device__ __forceinline__ void fence_mbar_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes,
-                                         uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-          "r"(smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase) {
-  const uint32_t a = smem_u32(bar);
-  for (uint32_t i = 0; i < kWaitLimit; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(a), "r"(phase)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void bulk_s2g(void* dst, const void* src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
-               "r"(smem_u32(src)), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit() {
-  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-__device__ __forceinline__ void bulk_wait_all() {
-  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-}
-
 // ---- warp reductions ------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-  return v;
-}
-template <typename T>
-__device__ __forceinline__ T warp_min(T v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const T w = __shfl_xor_sync(kFull, v, o);
-    v = w < v ? w : v;
-  }
-  return v;
-}
-template <typename T>
-__device__ __forceinline__ T warp_max(T v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const T w = __shfl_xor_sync(kFull, v, o);
-    v = w > v ? w : v;
-  }
   return v;
 }
 
@@ -202,7 +119,28 @@ __global__ void error_from_projection_kernel(const Real* __restrict__ y,
 // Per-view FP64 sums.  kind 0 (jointEstimation, HAADF_ReconstructionEngine_Extra.cpp:474-517):
 //   [0] sum y w, [1] sum w, [2] sum yh w, [3] sum yh w y, [4] sum y^2 w, [5] sum yh^2 w,
 //   yh = (y - e - mu)/I.  kind 1 (updateWeights :825-833): [0] sum e^2.
-template <typename Real, int K>
+//
+// The gain/offset solve subtracts these sums from one another and a sweep's zero skipping turns a
+// last-bit difference of its inputs into another path, so every rounding of the sums is kept.
+// The FP64 pipe bounds the kernel (2 lanes per clock and SM): kind 0 took ~23 FP64 operations per
+// entry, ~10 of them the division by the view's gain.  div_by gives the same quotient in five;
+// the FP32 engine leaves out sum y^2 w (Y2 false), which its solve does not use.
+
+// x / g, correctly rounded, from inv = rn(1 / g): one refinement makes the quotient faithful, a
+// second one correctly rounded (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990), for magnitudes far from the ends of the exponent range
+__device__ __forceinline__ bool mid_range(double x) {
+  const unsigned e = (static_cast<unsigned>(__double2hiint(x)) >> 20) & 0x7ffu;
+  return e - 400u < 1247u;  // 2^-623 <= |x| < 2^624
+}
+__device__ __forceinline__ double div_by(double x, double g, double inv, bool mid) {
+  if (!mid || !mid_range(x)) return x / g;
+  double q = x * inv;
+  q = fma(fma(-q, g, x), inv, q);
+  return fma(fma(-q, g, x), inv, q);
+}
+
+template <typename Real, int K, bool Y2>
 __global__ void view_sums_kernel(const Real* __restrict__ y, const Real* __restrict__ e,
                                  const double* __restrict__ mu, const double* __restrict__ gain,
                                  const double* __restrict__ wv, double* __restrict__ partial,
@@ -216,6 +154,9 @@ __global__ void view_sums_kernel(const Real* __restrict__ y, const Real* __restr
 #pragma unroll
   for (int k = 0; k < K; ++k) acc[k] = 0.0;
   const double m = mu[v], gi = gain[v], w = wv[v];
+  const double inv = K > 1 ? 1.0 / gi : 0.0;
+  // all of one mantissa bit pattern (all ones) is outside the theorem
+  const bool mid = mid_range(gi) && (__double_as_longlong(gi) & 0xfffffffffffffLL) != 0xfffffffffffffLL;
   for (int t = t0; t < t1; ++t) {
     const size_t base = (static_cast<size_t>(t) * n_theta + v) * n_rp;
     for (int r = threadIdx.x; r < n_r; r += blockDim.x) {
@@ -224,12 +165,12 @@ __global__ void view_sums_kernel(const Real* __restrict__ y, const Real* __restr
         acc[0] += ev * ev;
       } else {
         const double yv = y[base + r];
-        const double yh = (yv - ev - m) / gi;
+        const double yh = div_by(yv - ev - m, gi, inv, mid);
         acc[0] += yv * w;
         acc[1] += w;
         acc[2] += yh * w;
         acc[K > 3 ? 3 : 0] += yh * w * yv;
-        acc[K > 4 ? 4 : 0] += yv * yv * w;
+        if constexpr (Y2) acc[K > 4 ? 4 : 0] += yv * yv * w;
         acc[K > 5 ? 5 : 0] += yh * yh * w;
       }
     }
@@ -281,6 +222,44 @@ __global__ void rebuild_error_kernel(const Real* __restrict__ y, Real* __restric
   }
 }
 
+// rebuild_error_kernel of the FP32 engine: the same bits (mbir_wide.cuh)
+__global__ void __launch_bounds__(256)
+    rebuild_error_f32_kernel(const float* __restrict__ y, float* __restrict__ e,
+                             const double* __restrict__ mu_old, const double* __restrict__ gain_old,
+                             const double* __restrict__ mu_new, const double* __restrict__ gain_new,
+                             int n_theta, int n_rp, int n_r, int n_t, int n_chunk) {
+  const int v = blockIdx.x, ch = blockIdx.y;
+  const int t0 = static_cast<int>(static_cast<long long>(ch) * n_t / n_chunk);
+  const int t1 = static_cast<int>(static_cast<long long>(ch + 1) * n_t / n_chunk);
+  const double mo = mu_old[v], go = gain_old[v], mn = mu_new[v], gn = gain_new[v];
+  const wide::F2 mof = wide::neg(wide::split(mo)), mnf = wide::neg(wide::split(mn));
+  const wide::F2 ratio = wide::neg(wide::split(gn / go));
+  const float ra = fabsf(ratio.hi), fixed = fabsf(mnf.hi) + fabsf(mof.hi) * ra;
+  wide::for_view_rows(
+      v, t0, t1, n_theta, n_rp,
+      [&](size_t row, int r) {
+        const size_t base = row * n_rp;
+        const float4 y4 = *reinterpret_cast<const float4*>(y + base + r);
+        const float4 e4 = *reinterpret_cast<const float4*>(e + base + r);
+        const float yv[4] = {y4.x, y4.y, y4.z, y4.w}, ev[4] = {e4.x, e4.y, e4.z, e4.w};
+        float o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const wide::F2 d = wide::add(wide::two_diff(yv[j], ev[j]), mof);
+          const wide::F2 a = wide::add(wide::two_sum(yv[j], mnf.hi), wide::F2{mnf.lo, 0.f});
+          const float size = fabsf(yv[j]) * (1.f + ra) + fabsf(ev[j]) * ra + fixed;
+          if (!wide::rounds_to(wide::add(a, wide::mul(d, ratio)), 1.2e-13f * size, o[j])) {
+            const double yd = yv[j];
+            const double yh = (yd - static_cast<double>(ev[j]) - mo) / go;
+            o[j] = static_cast<float>(yd - mn - __dmul_rn(gn, yh));
+          }
+          if (r + j >= n_r) o[j] = ev[j];
+        }
+        *reinterpret_cast<float4*>(e + base + r) = make_float4(o[0], o[1], o[2], o[3]);
+      },
+      [](auto) {});
+}
+
 // QGGMRF prior term of computeCost (HAADF_ReconstructionEngine.cpp:1285-1359): 13 forward
 // neighbours per voxel, FP64 accumulation.  Offsets are (dz, dx, dy) with weight index
 // [dy+1][dz+1][dx+1].
@@ -288,43 +267,26 @@ __constant__ int c_fwd[13][3] = {{0, 0, 1},  {0, 1, -1}, {0, 1, 0},   {0, 1, 1},
                                  {1, 0, 0},  {1, 1, 0},  {1, -1, -1}, {1, -1, 1},  {1, 0, -1},
                                  {1, 1, -1}, {1, 1, 1},  {1, 0, 1}};
 
-template <typename Real>
-__global__ void prior_cost_kernel(const Real* __restrict__ x, DevFilter q, int n_z, int n_x,
+__global__ void prior_cost_kernel(const double* __restrict__ x, DevFilter q, int n_z, int n_x,
                                   int n_y, double* __restrict__ partial) {
   // one (y, z) row of n_x voxels at a time: 32-bit index arithmetic, coalesced row reads
   const int rows = n_y * n_z;
-  constexpr bool kF32 = std::is_same<Real, float>::value;
-  // FP32 engine: each voxel's 13 pair terms in FP32 (relative error ~1e-6 of the term),
-  // summed per voxel and accumulated in FP64; FP64 engine: FP64 throughout
-  const float P = static_cast<float>(q.mrf_p), PQ = static_cast<float>(q.mrf_p - q.mrf_q);
-  const float isp = static_cast<float>(1.0 / q.sig_p), ispq = static_cast<float>(1.0 / q.sig_pq);
-  const float cc = static_cast<float>(q.mrf_c);
-  const bool p2 = q.mrf_p == 2.0;
   double acc = 0.0;
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     const int yi = r / n_z, zi = r - yi * n_z;
-    const Real* row = x + static_cast<size_t>(r) * n_x;
+    const double* row = x + static_cast<size_t>(r) * n_x;
     for (int xi = threadIdx.x; xi < n_x; xi += blockDim.x) {
-      const Real c = row[xi];
-      float vsum = 0.f;
+      const double c = row[xi];
       for (int k = 0; k < 13; ++k) {
         const int zz = zi + c_fwd[k][0], xx = xi + c_fwd[k][1], yy = yi + c_fwd[k][2];
         if (zz < 0 || zz >= n_z || xx < 0 || xx >= n_x || yy < 0 || yy >= n_y) continue;
-        const Real nv = x[(static_cast<size_t>(yy) * n_z + zz) * n_x + xx];
+        const double nv = x[(static_cast<size_t>(yy) * n_z + zz) * n_x + xx];
         const int fi = 9 * (c_fwd[k][2] + 1) + 3 * (c_fwd[k][0] + 1) + (c_fwd[k][1] + 1);
-        if constexpr (kF32) {
-          const float ad = fabsf(c - nv);
-          const float num = p2 ? ad * ad : powf(ad, P);
-          const float pq = powf(ad, PQ);
-          vsum += static_cast<float>(q.f[fi]) * ((num * isp) / (cc + pq * ispq));
-        } else {
-          const double ad = fabs(static_cast<double>(c) - static_cast<double>(nv));
-          const double num = pow(ad, q.mrf_p);
-          const double pq = pow(ad, q.mrf_p - q.mrf_q);
-          acc += q.f[fi] * ((num / q.sig_p) / (q.mrf_c + pq / q.sig_pq));
-        }
+        const double ad = fabs(c - nv);
+        const double num = pow(ad, q.mrf_p);
+        const double pq = pow(ad, q.mrf_p - q.mrf_q);
+        acc += q.f[fi] * ((num / q.sig_p) / (q.mrf_c + pq / q.sig_pq));
       }
-      if constexpr (kF32) acc += static_cast<double>(vsum);
     }
   }
   acc = warp_sum(acc);
@@ -339,13 +301,57 @@ __global__ void prior_cost_kernel(const Real* __restrict__ x, DevFilter q, int n
   }
 }
 
+// The FP32 engine's: each voxel's 13 pair terms in FP32 (relative error ~1e-6 of the term),
+// summed per voxel and accumulated in FP64.  The pair weights are FP32 arguments (converted per
+// pair they took a third of the kernel on the FP64 pipe), and a pair of equal voxels adds nothing (its numerator is 0).
+struct PriorCostF {
+  float f[13];           // pair weights in c_fwd order
+  float P, PQ, isp, ispq, c;
+  int p2, skip_equal;
+};
+__global__ void __launch_bounds__(256)
+    prior_cost_f32_kernel(const float* __restrict__ x, const PriorCostF q, int n_z, int n_x,
+                          int n_y, double* __restrict__ partial) {
+  const int rows = n_y * n_z;
+  double acc = 0.0;
+  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+    const int yi = r / n_z, zi = r - yi * n_z;
+    const float* row = x + static_cast<size_t>(r) * n_x;
+    for (int xi = threadIdx.x; xi < n_x; xi += blockDim.x) {
+      const float c = row[xi];
+      float vsum = 0.f;
+      constexpr int fwd[13][3] = {{0, 0, 1},  {0, 1, -1}, {0, 1, 0},   {0, 1, 1},   {1, -1, 0},
+                                  {1, 0, 0},  {1, 1, 0},  {1, -1, -1}, {1, -1, 1},  {1, 0, -1},
+                                  {1, 1, -1}, {1, 1, 1},  {1, 0, 1}};  // c_fwd
+#pragma unroll
+      for (int k = 0; k < 13; ++k) {
+        const int xx = xi + fwd[k][1], yy = yi + fwd[k][2];
+        if (zi + fwd[k][0] >= n_z || yy < 0 || yy >= n_y) continue;  // (the same for the row)
+        if (xx < 0 || xx >= n_x) continue;
+        const float ad =
+            fabsf(c - row[(static_cast<long long>(fwd[k][2]) * n_z + fwd[k][0]) * n_x + xx]);
+        if (q.skip_equal && ad == 0.f) continue;
+        const float num = q.p2 ? ad * ad : powf(ad, q.P);
+        const float pq = powf(ad, q.PQ);
+        vsum += q.f[k] * ((num * q.isp) / (q.c + pq * q.ispq));
+      }
+      acc += static_cast<double>(vsum);
+    }
+  }
+  const double a1[1] = {acc};
+  const double s = wide::block_sums<1>(a1);
+  if (threadIdx.x == 0) partial[blockIdx.x] = s;
+}
+
+// One warp per column (the sums are of 2^-32 multiples below 2^21 or counts: exact in any order)
 __global__ void reduce_rows_kernel(const double* __restrict__ in, int n_rows, int n_cols,
                                    double* __restrict__ out) {
-  const int c = threadIdx.x;
+  const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (c >= n_cols) return;
   double s = 0.0;
-  for (int r = 0; r < n_rows; ++r) s += in[static_cast<size_t>(r) * n_cols + c];
-  out[c] = s;
+  for (int r = lane; r < n_rows; r += 32) s += in[static_cast<size_t>(r) * n_cols + c];
+  s = warp_sum(s);
+  if (lane == 0) out[c] = s;
 }
 
 inline int ok_or(cudaError_t e) { return e == cudaSuccess ? 0 : -3; }
@@ -466,30 +472,33 @@ int launch_view_sums(int kind, const void* y, const void* e, const double* mu,
                      int n_theta, int n_rp, int n_r, int n_t, int n_chunk, int fp64,
                      void* stream) {
   return launch_view_sums_rows(kind, y, e, mu, gain, wv, partial, out, n_theta, n_rp, n_r, 0, n_t,
-                               n_chunk, fp64, stream);
+                               n_chunk, fp64, false, stream);
 }
 
 int launch_view_sums_rows(int kind, const void* y, const void* e, const double* mu,
                           const double* gain, const double* wv, double* partial, double* out,
                           int n_theta, int n_rp, int n_r, int t_begin, int t_end, int n_chunk,
-                          int fp64, void* stream) {
+                          int fp64, bool all_sums, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   dim3 grid(n_theta, n_chunk);
   const int K = kind == 0 ? 6 : 1;
+  auto go = [&](auto kern, auto zero) {
+    using Real = decltype(zero);
+    kern<<<grid, 256, 0, s>>>(RP<Real>(y), RP<Real>(e), mu, gain, wv, partial, n_theta, n_rp, n_r,
+                              t_begin, t_end, n_chunk);
+  };
   if (fp64) {
     if (kind == 0)
-      view_sums_kernel<double, 6><<<grid, 256, 0, s>>>(RP<double>(y), RP<double>(e), mu, gain, wv,
-                                                        partial, n_theta, n_rp, n_r, t_begin, t_end, n_chunk);
+      go(view_sums_kernel<double, 6, true>, 0.0);
     else
-      view_sums_kernel<double, 1><<<grid, 256, 0, s>>>(RP<double>(y), RP<double>(e), mu, gain, wv,
-                                                        partial, n_theta, n_rp, n_r, t_begin, t_end, n_chunk);
+      go(view_sums_kernel<double, 1, false>, 0.0);
+  } else if (kind == 0) {
+    if (all_sums)
+      go(view_sums_kernel<float, 6, true>, 0.f);
+    else
+      go(view_sums_kernel<float, 6, false>, 0.f);
   } else {
-    if (kind == 0)
-      view_sums_kernel<float, 6><<<grid, 256, 0, s>>>(RP<float>(y), RP<float>(e), mu, gain, wv,
-                                                       partial, n_theta, n_rp, n_r, t_begin, t_end, n_chunk);
-    else
-      view_sums_kernel<float, 1><<<grid, 256, 0, s>>>(RP<float>(y), RP<float>(e), mu, gain, wv,
-                                                       partial, n_theta, n_rp, n_r, t_begin, t_end, n_chunk);
+    go(view_sums_kernel<float, 1, false>, 0.f);
   }
   const int n = n_theta * K;
   view_sums_final_kernel<<<(n + 127) / 128, 128, 0, s>>>(partial, out, n_theta, n_chunk, K);
@@ -504,21 +513,38 @@ int launch_rebuild_error(const void* y, void* e, const double* mu_old, const dou
     rebuild_error_kernel<double><<<grid_for(n, 256), 256, 0, s>>>(
         RP<double>(y), RP<double>(e), mu_old, gain_old, mu_new, gain_new, n_theta, n_rp, n_r, n_t);
   else
-    rebuild_error_kernel<float><<<grid_for(n, 256), 256, 0, s>>>(
-        RP<float>(y), RP<float>(e), mu_old, gain_old, mu_new, gain_new, n_theta, n_rp, n_r, n_t);
+    rebuild_error_f32_kernel<<<dim3(n_theta, std::min(32, n_t)), 256, 0, s>>>(
+        RP<float>(y), RP<float>(e), mu_old, gain_old, mu_new, gain_new, n_theta, n_rp, n_r, n_t,
+        std::min(32, n_t));
   return ok_or(cudaGetLastError());
 }
 int launch_prior_cost(const void* x, const DevFilter& f, int n_z, int n_x, int n_y,
                       double* partial, int n_blocks, int fp64, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (fp64)
-    prior_cost_kernel<double><<<n_blocks, 256, 0, s>>>(RP<double>(x), f, n_z, n_x, n_y, partial);
-  else
-    prior_cost_kernel<float><<<n_blocks, 256, 0, s>>>(RP<float>(x), f, n_z, n_x, n_y, partial);
+    prior_cost_kernel<<<n_blocks, 256, 0, s>>>(RP<double>(x), f, n_z, n_x, n_y, partial);
+  else {
+    PriorCostF q{};
+    constexpr int fwd[13][3] = {{0, 0, 1},  {0, 1, -1}, {0, 1, 0},   {0, 1, 1},   {1, -1, 0},
+                                {1, 0, 0},  {1, 1, 0},  {1, -1, -1}, {1, -1, 1},  {1, 0, -1},
+                                {1, 1, -1}, {1, 1, 1},  {1, 0, 1}};  // c_fwd
+    for (int k = 0; k < 13; k++)
+      q.f[k] = static_cast<float>(f.f[9 * (fwd[k][2] + 1) + 3 * (fwd[k][0] + 1) + fwd[k][1] + 1]);
+    q.P = static_cast<float>(f.mrf_p);
+    q.PQ = static_cast<float>(f.mrf_p - f.mrf_q);
+    q.isp = static_cast<float>(1.0 / f.sig_p);
+    q.ispq = static_cast<float>(1.0 / f.sig_pq);
+    q.c = static_cast<float>(f.mrf_c);
+    q.p2 = f.mrf_p == 2.0 ? 1 : 0;
+    // a pair of equal voxels: 0 / c, or 0 / inf, unless the constants make it 0 / 0 or inf 0
+    q.skip_equal = f.mrf_p > 0 && q.c > 0.f && q.isp <= 3e38f && q.ispq >= 0.f ? 1 : 0;
+    prior_cost_f32_kernel<<<n_blocks, 256, 0, s>>>(RP<float>(x), q, n_z, n_x, n_y, partial);
+  }
   return ok_or(cudaGetLastError());
 }
 int launch_reduce_stats(const double* in, int n_rows, int n_cols, double* out, void* stream) {
-  reduce_rows_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(in, n_rows, n_cols, out);
+  reduce_rows_kernel<<<1, 32 * n_cols, 0, static_cast<cudaStream_t>(stream)>>>(in, n_rows, n_cols,
+                                                                              out);
   return ok_or(cudaGetLastError());
 }
 

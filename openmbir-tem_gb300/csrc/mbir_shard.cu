@@ -169,7 +169,7 @@ int Engine::view_sums(int kind, double* out) {
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   int rc = launch_view_sums_rows(kind, d_y_, d_e_, d_mu_, d_gain_, d_wv_, d_partial_, d_vsum_, nt,
-                                 n_rp_, g.n_r, t0, t1, n_chunk_, fp64_, s);
+                                 n_rp_, g.n_r, t0, t1, n_chunk_, fp64_, true, s);
   if (rc) return cuda_check(rc, "view sums");
   cudaMemcpyAsync(out, d_vsum_, sizeof(double) * nt * K, cudaMemcpyDeviceToHost, s);
   return cudaStreamSynchronize(s) == cudaSuccess ? MBIR_OK : cuda_check(MBIR_EDEVICE, "view sums");
@@ -306,7 +306,7 @@ int Engine::bf_slab_sums(int kind, double* out) {
     cudaMemcpyAsync(out, d_vsum_, sizeof(double) * K, cudaMemcpyDeviceToHost, s);
   } else {
     cudaMemcpyAsync(d_alpha_, alpha_.data(), sizeof(double) * nt, cudaMemcpyHostToDevice, s);
-    rc = launch_bf_variance_sums(b, 0, d_alpha_, d_bfpart_, d_bfout_, s);
+    rc = launch_bf_variance_sums(b, 0, d_alpha_, true, d_bfpart_, d_bfout_, s);
     if (rc) return cuda_check(rc, "variance sums");
     cudaMemcpyAsync(out, d_bfout_, sizeof(double) * 2, cudaMemcpyDeviceToHost, s);
     out[2] = static_cast<double>(nt) * g_.n_r * (t1 - t0);
