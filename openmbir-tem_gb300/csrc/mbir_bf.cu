@@ -549,6 +549,126 @@ __global__ void vsc_kernel(const double* __restrict__ mag, double* __restrict__ 
   filt[idx] = f;
 }
 
+// The lines of a homogeneous call: active mask, and their magnitudes restart at 0
+__global__ void h_list_kernel(const uint8_t* __restrict__ slot, int j, uint8_t* __restrict__ active,
+                              unsigned long long* __restrict__ fx, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const bool on = slot[i] == j;
+  active[i] = on ? 1 : 0;
+  if (on) fx[i] = 0ull;
+}
+
+// The lines of a non-homogeneous call (SetNonHomThreshold, GenNonHomList): those whose filtered
+// magnitude exceeds the order statistic `rank` (0-based, ascending).  One CTA: the order
+// statistic by radix selection on the bits of the (non-negative) magnitudes, 8 at a time from
+// the top, until the bucket holds at most kTail values, which are then ranked directly; then the
+// active mask, the magnitudes' restart and the ascending list of the active lines with an
+// A-column.  On the host (read-back of the map, nth_element, list, upload) this took ~0.25 ms of
+// a call's 2.1 on 512 x 128 lines; here ~0.03.
+constexpr int kTail = 1024;
+__global__ void __launch_bounds__(1024)
+    nh_list_kernel(const double* __restrict__ filt, const uint8_t* __restrict__ lineok, int n,
+                   int rank, uint8_t* __restrict__ active, unsigned long long* __restrict__ fx,
+                   int* __restrict__ vis, int* __restrict__ n_vis) {
+  __shared__ int hist[256];
+  __shared__ unsigned long long tail[kTail];
+  __shared__ unsigned long long s_prefix;
+  __shared__ int s_rank, s_count, s_n;
+  __shared__ int warp_n[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned long long* bits = reinterpret_cast<const unsigned long long*>(filt);
+  unsigned long long prefix = 0ull;  // the bits above `shift + 8` of the order statistic
+  int r = rank, count = n, shift = 64;
+  while (count > kTail && shift > 0) {
+    shift -= 8;
+    if (tid < 256) hist[tid] = 0;
+    __syncthreads();
+    for (int i0 = 0; i0 < n; i0 += 1024) {
+      const int i = i0 + tid;
+      const unsigned long long v = i < n ? bits[i] : 0ull;
+      const bool in = i < n && (shift == 56 || (v >> (shift + 8)) == prefix);
+      const int d = in ? static_cast<int>((v >> shift) & 255u) : -1;
+      // the values of a warp share their upper digits: one addition per distinct digit
+      const unsigned same = __match_any_sync(0xffffffffu, d);
+      if (in && lane == __ffs(same) - 1) atomicAdd(&hist[d], __popc(same));
+    }
+    __syncthreads();
+    if (warp == 0) {  // the bucket of rank r: eight digits per lane, summed across the warp
+      int c[8], t = 0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        c[k] = hist[8 * lane + k];
+        t += c[k];
+      }
+      int before = t;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += u;
+      }
+      before -= t;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        if (r >= before && r < before + c[k]) {
+          s_prefix = (prefix << 8) | static_cast<unsigned>(8 * lane + k);
+          s_rank = r - before;
+          s_count = c[k];
+        }
+        before += c[k];
+      }
+    }
+    __syncthreads();
+    prefix = s_prefix;
+    r = s_rank;
+    count = s_count;
+    __syncthreads();
+  }
+  if (shift > 0) {  // rank the bucket's values
+    if (tid == 0) s_n = 0;
+    __syncthreads();
+    for (int i = tid; i < n; i += 1024) {
+      const unsigned long long v = bits[i];
+      if (shift == 64 || (v >> shift) == prefix) tail[atomicAdd(&s_n, 1)] = v;
+    }
+    __syncthreads();
+    if (tid < count) {
+      const unsigned long long v = tail[tid];
+      int less = 0, same = 0;
+      for (int k = 0; k < count; ++k) {
+        less += tail[k] < v;
+        same += tail[k] == v;
+      }
+      if (less <= r && r < less + same) s_prefix = v;
+    }
+    __syncthreads();
+    prefix = s_prefix;
+  }
+  const double thr = __longlong_as_double(static_cast<long long>(prefix));
+  int base = 0;
+  for (int i0 = 0; i0 < n; i0 += 1024) {
+    const int i = i0 + tid;
+    const bool on = i < n && filt[i] > thr;
+    if (i < n) {
+      active[i] = on ? 1 : 0;
+      if (on) fx[i] = 0ull;
+    }
+    const bool in = on && lineok[i] != 0;
+    const unsigned b = __ballot_sync(0xffffffffu, in);
+    if (lane == 0) warp_n[warp] = __popc(b);
+    __syncthreads();
+    int at = base + __popc(b & ((1u << lane) - 1u)), all = 0;
+    for (int w = 0; w < 32; ++w) {
+      at += w < warp ? warp_n[w] : 0;
+      all += warp_n[w];
+    }
+    if (in) vis[at] = i;
+    base += all;
+    __syncthreads();
+  }
+  if (tid == 0) *n_vis = base;
+}
+
 __global__ void nh_mask_kernel(const double* __restrict__ filt, double thr,
                                uint8_t* __restrict__ active, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -763,6 +883,20 @@ int launch_bf_mag_update(const unsigned long long* fx, const uint8_t* active, do
 int launch_bf_vsc(const double* mag, double* filt, int n_z, int n_x, void* stream) {
   const int n = n_z * n_x;
   vsc_kernel<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(mag, filt, n_z, n_x);
+  return ok_or(cudaGetLastError());
+}
+
+int launch_bf_h_list(const uint8_t* slot, int j, uint8_t* active, unsigned long long* fx, int n,
+                     void* stream) {
+  h_list_kernel<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(slot, j, active, fx,
+                                                                               n);
+  return ok_or(cudaGetLastError());
+}
+
+int launch_bf_nh_list(const double* filt, const uint8_t* lineok, int n, int rank, uint8_t* active,
+                      unsigned long long* fx, int* vis, int* n_vis, void* stream) {
+  nh_list_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(filt, lineok, n, rank, active,
+                                                                    fx, vis, n_vis);
   return ok_or(cudaGetLastError());
 }
 

@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kThreads) colour_conflicts_kernel(ColourArgs A
   __shared__ int vz[(kBack + 1) * kBlock], vx[(kBack + 1) * kBlock];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int bk = blockIdx.x, s = bk * kBlock;
-  const int m = min(kBlock, A.n - s);
+  const int m = min(kBlock, (A.n_dev ? *A.n_dev : A.n) - s);
   if (m <= 0) return;
   for (int r = warp; r < (kBack + 1) * kBlock; r += kThreads / 32) {
     const int d = r / kBlock, j = r - d * kBlock;  // block bk - d, line j
@@ -270,7 +270,7 @@ __device__ int wait_flag(const ColourArgs& A, const int* flag) {
 // Helper CTA of the multi-CTA form: the taken-colour sets of its blocks (read from the planes
 // once the blocks up to b-kBack-1 are in them), then its blocks' colours into the planes.
 __device__ void colour_helper(const ColourArgs& A, unsigned char* smem) {
-  const int W = A.words, nt = A.n_theta, n = A.n;
+  const int W = A.words, nt = A.n_theta, n = A.n_dev ? *A.n_dev : A.n;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nblk = (n + kBlock - 1) / kBlock;
   int* ready = A.flags;
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(kThreads, 1) colour_kernel(ColourArgs A) {
     s_fail = 0;
 
   }
-  const int n = A.n;  // the call's lines, ascending, in A.vis
+  const int n = A.n_dev ? *A.n_dev : A.n;  // the call's lines, ascending, in A.vis
   __syncthreads();
 
   // phase 1: colour kBlock lines per step; block 0's lines need no planes (nothing coloured)

@@ -150,6 +150,11 @@ void Engine::release() {
   dfree(d_hc_lines_);
   dfree(d_hc_lofs_);
   dfree(d_hc_count_);
+  dfree(d_slot_);
+  dfree(d_hvis_);
+  dfree(d_nvis_);
+  dev_lists_ = false;
+  lists_stale_ = false;
   hc_valid_.clear();
   sched_ready_ = false;
   acol_lo_.clear();
@@ -671,7 +676,7 @@ int Engine::alloc_device() {
   rc |= dmalloc(&d_Href_, static_cast<size_t>(g.n_theta) * bins_);
   rc |= dmalloc(&d_lines_, static_cast<size_t>(g.n_z) * g.n_x);
   rc |= dmalloc(&d_stats_, static_cast<size_t>((g.n_y + 1) / 2 + 1) * kStatSlots * 2);
-  rc |= dmalloc(&d_stat4_, kStatSlots);
+  rc |= dmalloc_bytes(reinterpret_cast<void**>(&d_stat4_), sizeof(SweepResult));
   rc |= dmalloc(&d_mu2_, g.n_theta);
   rc |= dmalloc(&d_gain2_, g.n_theta);
   n_chunk_ = std::min(32, std::max(1, g.n_t));
@@ -749,7 +754,12 @@ int Engine::check_device_error() {
   if (cudaMemcpyAsync(&h, d_err_, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return cuda_check(MBIR_EDEVICE, "device error check");
+  return device_error(h);
+}
+
+int Engine::device_error(int h) {
   if (h == 0) return 0;
+  cudaStream_t s = static_cast<cudaStream_t>(stream_);
   // reported once: the work a timed-out wait guarded was skipped, the state stays consistent
   cudaMemsetAsync(d_err_, 0, sizeof(int), s);
   if (h & 4)
@@ -1215,14 +1225,16 @@ int Engine::sweep(int outer, int inner, double* stats4) {
     }
     cudaEventRecord(static_cast<cudaEvent_t>(ev3_), s);
     kernel_timed_ = true;
-    if ((rc = launch_reduce_stats(d_stats_, g.n_y, kStatSlots, d_stat4_, s)))
+    if ((rc = launch_reduce_stats(d_stats_, g.n_y, kStatSlots, d_stat4_, s, d_err_)))
       return cuda_check(rc, "stats reduce");
   }
   cudaEventRecord(static_cast<cudaEvent_t>(ev1_), s);
-  double st[kStatSlots];
-  cudaMemcpyAsync(st, d_stat4_, sizeof(st), cudaMemcpyDeviceToHost, s);
+  SweepResult res{};
+  const bool walked = p_.order_mode != MBIR_ORDER_REFERENCE;  // the error word came along
+  cudaMemcpyAsync(&res, d_stat4_, walked ? sizeof(res) : sizeof(res.stat), cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "ICD sweep");
-  if ((rc = check_device_error())) return rc;
+  if ((rc = walked ? device_error(res.err) : check_device_error())) return rc;
+  const double* st = res.stat;
   float ms = 0;
   cudaEventElapsedTime(&ms, static_cast<cudaEvent_t>(ev0_), static_cast<cudaEvent_t>(ev1_));
   icd_ms_ += ms;
@@ -1312,6 +1324,7 @@ int Engine::batch_args(int outer, int inner, SweepArgs* out) {
 
 int Engine::batch_finish(int outer, int inner, const double* st, double ms) {
   if (bf_) {
+    bf_schedule_readback();
     int rc = bf_call_end();
     if (rc) return rc;
     if (cudaStreamSynchronize(static_cast<cudaStream_t>(stream_)) != cudaSuccess)

@@ -218,6 +218,9 @@ class Engine {
   int alloc_device();
   int upload_views();  // (gain, weight) pairs and mu/gain doubles
   int check_device_error();
+  int device_error(int h);
+  int bf_call_begin_device(DevBF* out);
+  int fetch_call_lists();
   void row_order_for_sweep(int sweep, std::vector<int32_t>& order) const;
   ExactArgs exact_args();
   int cuda_check(int code, const char* what);
@@ -299,7 +302,7 @@ class Engine {
   double* d_Href_ = nullptr;
   int* d_lines_ = nullptr;
   double* d_stats_ = nullptr;   // [max slices][4]
-  double* d_stat4_ = nullptr;   // [4]
+  double* d_stat4_ = nullptr;   // SweepResult
   double* d_mu_ = nullptr;      // [n_theta]
   double* d_gain_ = nullptr;
   double* d_mu2_ = nullptr;
@@ -349,6 +352,15 @@ class Engine {
   std::vector<int32_t> bf_master_;          // random permutation of all lines
   std::vector<int32_t> call_lines_;         // lines of the last sweep/call
   std::vector<uint8_t> active_host_;
+  // device lists of scheduled calls: each line's homogeneous sub-list, the sub-lists' lines
+  // (ascending, with an A-column) and where they start, the last non-homogeneous call's length
+  bool dev_lists_ = false;
+  uint8_t* d_slot_ = nullptr;
+  int32_t* d_hvis_ = nullptr;
+  int32_t* d_nvis_ = nullptr;
+  std::vector<int> hvis_start_;
+  int active_bound_ = 0;                    // at most this many lines in the non-homogeneous call
+  mutable bool lists_stale_ = false;        // call_lines_, sched_lines_, sched_lofs_: on the device
   uint32_t bf_listsel_ = 0, bf_eff_ = 0;
   int slab_y0_ = 0, slab_y1_ = 0;           // 0, 0: the whole volume
   bool slab_call_open_ = false;             // a bright-field slab call between begin and end

@@ -212,6 +212,36 @@ int Engine::bf_prepare_schedule() {
   }
   hc_valid_.assign(kNumHomogeneous, 0);
   hc_start_.assign(kNumHomogeneous, 0);
+  // the sub-lists on the device (without them each call's lines come from the host)
+  if (cudaMalloc(&d_slot_, nl) != cudaSuccess ||
+      cudaMalloc(&d_hvis_, nl * sizeof(int32_t)) != cudaSuccess ||
+      cudaMalloc(&d_nvis_, sizeof(int32_t)) != cudaSuccess) {
+    cudaGetLastError();
+    dfree_any(d_slot_);
+    dfree_any(d_hvis_);
+    dfree_any(d_nvis_);
+  } else {
+    const int per = static_cast<int>(nl) / kNumHomogeneous;
+    std::vector<uint8_t> slot(nl);
+    std::vector<int> len(kNumHomogeneous, 0);
+    for (size_t i = 0; i < nl; i++) {
+      const int j = per > 0 ? std::min(static_cast<int>(i) / per, kNumHomogeneous - 1)
+                            : kNumHomogeneous - 1;
+      const int32_t l = bf_master_[i];
+      slot[l] = static_cast<uint8_t>(j);
+      if (tab_.line_nonempty[l]) len[j]++;
+    }
+    hvis_start_.assign(kNumHomogeneous + 1, 0);
+    for (int j = 0; j < kNumHomogeneous; j++) hvis_start_[j + 1] = hvis_start_[j] + len[j];
+    std::vector<int> at(hvis_start_.begin(), hvis_start_.end() - 1);
+    std::vector<int32_t> vis(nl);
+    for (size_t l = 0; l < nl; l++)
+      if (tab_.line_nonempty[l]) vis[at[slot[l]]++] = static_cast<int32_t>(l);
+    cudaMemcpyAsync(d_slot_, slot.data(), nl, cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(d_hvis_, vis.data(), nl * sizeof(int32_t), cudaMemcpyHostToDevice, s);
+    if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "call lists");
+    dev_lists_ = true;
+  }
   if ((rc = launch_pack_footprints(d_acol_, n_entries, nb_, d_packed_, s)))
     return cuda_check(rc, "packed bins");
   if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "packed bins");
@@ -263,6 +293,7 @@ int Engine::bf_schedule(const std::vector<int32_t>& rows, SweepArgs& a) {
     rb_lofs_ = out_lofs;
     rb_count_ = out_count;
     sched_on_device_ = true;
+    lists_stale_ = true;
     a.sched_lines = out_lines;
     a.sched_lofs = out_lofs;
     a.sched_count = out_count;
@@ -282,14 +313,23 @@ int Engine::bf_schedule(const std::vector<int32_t>& rows, SweepArgs& a) {
     ca.lineok = d_lineok_;
     ca.active = d_active_;
     // the call's lines (lineok and active), ascending
-    vis_host_.clear();
-    for (size_t l = 0; l < active_host_.size(); ++l)
-      if (active_host_[l] && tab_.line_nonempty[l]) vis_host_.push_back(static_cast<int32_t>(l));
-    if (!vis_host_.empty())
-      cudaMemcpyAsync(d_vis_, vis_host_.data(), vis_host_.size() * sizeof(int32_t),
-                      cudaMemcpyHostToDevice, s);
-    ca.vis = d_vis_;
-    ca.n = static_cast<int>(vis_host_.size());
+    if (dev_lists_ && cur_hslot_ >= 0) {
+      ca.vis = d_hvis_ + hvis_start_[cur_hslot_];
+      ca.n = hvis_start_[cur_hslot_ + 1] - hvis_start_[cur_hslot_];
+    } else if (dev_lists_) {  // fewer than 1/20 of the lines lie above the order statistic
+      ca.vis = d_vis_;
+      ca.n = static_cast<int>(active_bound_);
+      ca.n_dev = d_nvis_;
+    } else {
+      vis_host_.clear();
+      for (size_t l = 0; l < active_host_.size(); ++l)
+        if (active_host_[l] && tab_.line_nonempty[l]) vis_host_.push_back(static_cast<int32_t>(l));
+      if (!vis_host_.empty())
+        cudaMemcpyAsync(d_vis_, vis_host_.data(), vis_host_.size() * sizeof(int32_t),
+                        cudaMemcpyHostToDevice, s);
+      ca.vis = d_vis_;
+      ca.n = static_cast<int>(vis_host_.size());
+    }
     ca.conf = d_conf_;
     ca.conf_p1 = d_conf_ + static_cast<size_t>(g.n_z) * g.n_x;
     ca.conf_p2 = d_conf_ + 2 * static_cast<size_t>(g.n_z) * g.n_x;
@@ -342,6 +382,7 @@ int Engine::bf_schedule(const std::vector<int32_t>& rows, SweepArgs& a) {
   if (levels == -2) levels = level_schedule(in, sched_work_, sched_lines_, sched_lofs_);
   if (levels < 0) return fail(MBIR_EINVAL, "call schedule: invalid row order");
   call_lines_ = sched_lines_;
+  lists_stale_ = false;
   sched_ms_ += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0)
                    .count();
   n_levels_ = levels;
@@ -365,6 +406,7 @@ int Engine::bf_schedule(const std::vector<int32_t>& rows, SweepArgs& a) {
 int Engine::bf_call_begin(int outer, int inner, DevBF* out) {
   (void)outer;
   (void)inner;
+  if (dev_lists_) return bf_call_begin_device(out);
   const Geometry& g = g_;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   const int nl = g.n_z * g.n_x;
@@ -436,23 +478,71 @@ int Engine::bf_call_begin(int outer, int inner, DevBF* out) {
   return MBIR_OK;
 }
 
-// The device schedule's lines, offsets and counts, copied to the host behind the call (the
-// caller synchronises the stream before bf_schedule_settle).
-void Engine::bf_schedule_readback() {
-  readback_pending_ = false;
-  if (!sched_on_device_) return;
+// The same with the lists on the device, for calls that are scheduled there: nothing is copied
+// and nothing waited for.  The host's copies of a call's lines are fetched when they are asked
+// for (fetch_call_lists).
+int Engine::bf_call_begin_device(DevBF* out) {
+  const Geometry& g = g_;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  size_t n_call = 0;
-  for (size_t l = 0; l < active_host_.size(); ++l)
-    n_call += (active_host_[l] && tab_.line_nonempty[l]) ? 1 : 0;
-  call_lines_.assign(n_call, 0);
-  sched_lofs_.assign(lofs_cap(), 0);
-  if (n_call)
-    cudaMemcpyAsync(call_lines_.data(), rb_lines_, n_call * sizeof(int32_t),
+  const int nl = g.n_z * g.n_x;
+  int rc;
+  cur_hslot_ = -1;
+  if (bf_eff_ % 2 == 0) {
+    bf_listsel_ %= kNumHomogeneous;
+    cur_hslot_ = static_cast<int>(bf_listsel_);
+    hc_start_[cur_hslot_] = nl / kNumHomogeneous * cur_hslot_;
+    bf_listsel_++;
+    if ((rc = launch_bf_h_list(d_slot_, cur_hslot_, d_active_, d_magfx_, nl, s)))
+      return cuda_check(rc, "call lines");
+  } else {
+    if ((rc = launch_bf_vsc(d_mag_, d_filt_, g.n_z, g.n_x, s))) return cuda_check(rc, "VSC filter");
+    int k = nl - nl / kNumNonHomogeneous;
+    if (k >= nl) k = nl - 1;
+    active_bound_ = nl - 1 - k;
+    if ((rc = launch_bf_nh_list(d_filt_, d_lineok_, nl, k, d_active_, d_magfx_, d_vis_, d_nvis_, s)))
+      return cuda_check(rc, "call lines");
+  }
+  if (out) {
+    out->w = d_w_;
+    out->sel = d_sel_;
+    out->n_sp = n_sp_;
+    out->active = d_active_;
+    out->mag_fx = d_magfx_;
+    out->bragg_t = bragg_t_;
+    out->bragg_dt = p_.bragg_delta * bragg_t_;
+  }
+  return MBIR_OK;
+}
+
+// The last device-scheduled call's lines and class offsets on the host (get_call_lines,
+// get_call_schedule)
+int Engine::fetch_call_lists() {
+  if (!lists_stale_) return MBIR_OK;
+  cudaStream_t s = static_cast<cudaStream_t>(stream_);
+  int32_t count[2] = {0, 0};
+  cudaMemcpyAsync(count, rb_count_, sizeof(count), cudaMemcpyDeviceToHost, s);
+  if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "call schedule");
+  call_lines_.assign(static_cast<size_t>(std::max(count[0], 0)), 0);
+  sched_lofs_.assign(static_cast<size_t>(std::max(count[1], 0)) + 1, 0);
+  if (!call_lines_.empty())
+    cudaMemcpyAsync(call_lines_.data(), rb_lines_, call_lines_.size() * sizeof(int32_t),
                     cudaMemcpyDeviceToHost, s);
   cudaMemcpyAsync(sched_lofs_.data(), rb_lofs_, sched_lofs_.size() * sizeof(int32_t),
                   cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(sched_count_host_, rb_count_, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
+  if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "call schedule");
+  sched_lines_ = call_lines_;
+  n_levels_ = count[1];
+  lists_stale_ = false;
+  return MBIR_OK;
+}
+
+// The device schedule's counts, copied to the host behind the call (the caller synchronises the
+// stream before bf_schedule_settle).
+void Engine::bf_schedule_readback() {
+  readback_pending_ = false;
+  if (!sched_on_device_) return;
+  cudaMemcpyAsync(sched_count_host_, rb_count_, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost,
+                  static_cast<cudaStream_t>(stream_));
   readback_pending_ = true;
 }
 
@@ -472,14 +562,9 @@ void Engine::bf_schedule_settle() {
   if (!readback_pending_) return;
   readback_pending_ = false;
   n_levels_ = sched_count_host_[1];
-  if (sched_count_host_[0] >= 0 && static_cast<size_t>(sched_count_host_[0]) <= call_lines_.size())
-    call_lines_.resize(static_cast<size_t>(sched_count_host_[0]));
-  sched_lofs_.resize(static_cast<size_t>(std::max(n_levels_, 0)) + 1);
-  sched_lines_ = call_lines_;
 }
 
 int Engine::bf_call_end() {
-  bf_schedule_readback();
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   const int nl = g_.n_z * g_.n_x;
   if (!exact_) {
@@ -552,16 +637,24 @@ int Engine::bf_call(int outer, int inner, double* st4) {
     }
     cudaEventRecord(static_cast<cudaEvent_t>(ev3_), s);
     kernel_timed_ = true;
-    if ((rc = launch_reduce_stats(d_stats_, g.n_y, kStatSlots, d_stat4_, s)))
+    if ((rc = launch_reduce_stats(d_stats_, g.n_y, kStatSlots, d_stat4_, s, d_err_,
+                                  sched_on_device_ ? rb_count_ : nullptr)))
       return cuda_check(rc, "stats reduce");
   }
   cudaEventRecord(static_cast<cudaEvent_t>(ev1_), s);
   if ((rc = bf_call_end())) return rc;
-  double st[kStatSlots];
-  cudaMemcpyAsync(st, d_stat4_, sizeof(st), cudaMemcpyDeviceToHost, s);
+  SweepResult res{};
+  const bool walked = p_.order_mode != MBIR_ORDER_REFERENCE;  // error word and counts came along
+  cudaMemcpyAsync(&res, d_stat4_, walked ? sizeof(res) : sizeof(res.stat), cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "BF call");
+  if (walked && sched_on_device_) {
+    sched_count_host_[0] = res.count[0];
+    sched_count_host_[1] = res.count[1];
+    readback_pending_ = true;
+  }
   bf_schedule_settle();
-  if ((rc = check_device_error())) return rc;
+  if ((rc = walked ? device_error(res.err) : check_device_error())) return rc;
+  const double* st = res.stat;
   float ms = 0;
   cudaEventElapsedTime(&ms, static_cast<cudaEvent_t>(ev0_), static_cast<cudaEvent_t>(ev1_));
   icd_ms_ += ms;
@@ -585,8 +678,10 @@ int Engine::bf_parallel_args(int iter_nonzero, const DevBF& bfa, SweepArgs* out,
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   int rc;
   std::vector<int32_t> rows;
-  row_order_for_sweep(sweeps_done_, rows);
-  cudaMemcpyAsync(d_rows_, rows.data(), sizeof(int) * g.n_z, cudaMemcpyHostToDevice, s);
+  if (!dev_lists_) {  // (calls scheduled on the device walk no rows)
+    row_order_for_sweep(sweeps_done_, rows);
+    cudaMemcpyAsync(d_rows_, rows.data(), sizeof(int) * g.n_z, cudaMemcpyHostToDevice, s);
+  }
   SweepArgs& a = *out;
   a = SweepArgs{};
   a.g = dg_;
@@ -786,6 +881,7 @@ int Engine::bf_run() {
 
 int Engine::get_call_schedule(int32_t* lines, int32_t cap, int32_t* lofs, int32_t lofs_cap,
                               int32_t* n_lines, int32_t* n_levels) const {
+  if (int rc = const_cast<Engine*>(this)->fetch_call_lists()) return rc;
   const bool sched = !sched_lofs_.empty() && n_levels_ > 0;
   const size_t nlev = sched ? sched_lofs_.size() - 1 : 0;
   if (n_lines) *n_lines = sched ? static_cast<int32_t>(sched_lines_.size()) : 0;
@@ -814,6 +910,7 @@ int Engine::get_footprint_bins(int16_t* lo, uint16_t* mask, uint8_t* lineok) con
 }
 
 int Engine::get_call_lines(int32_t* lines, int32_t cap, int32_t* n) const {
+  if (int rc = const_cast<Engine*>(this)->fetch_call_lists()) return rc;
   if (n) *n = static_cast<int32_t>(call_lines_.size());
   if (lines) {
     if (cap < static_cast<int32_t>(call_lines_.size())) return MBIR_EINVAL;

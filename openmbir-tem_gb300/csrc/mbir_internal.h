@@ -184,7 +184,8 @@ struct ColourArgs {
   const uint8_t* lineok;          // [n_z*n_x]
   const uint8_t* active;          // [n_z*n_x] lines of the call (nullptr: all)
   const int32_t* vis;             // [n] the call's lines (lineok and active), ascending
-  int n;
+  int n;                          // (with n_dev: at most)
+  const int32_t* n_dev;           // their number on the device, or nullptr
   unsigned* conf;                 // [n] scratch: conflict words of each block of 32 lines
   unsigned* conf_p1;              // [n] scratch: conflict words against the block before
   unsigned* conf_p2;              // [n] scratch: against the block before that
@@ -312,6 +313,11 @@ int launch_bf_mag_reset(unsigned long long* fx, const uint8_t* active, int n, vo
 int launch_bf_mag_update(const unsigned long long* fx, const uint8_t* active, double* mag, int n,
                          void* stream);
 int launch_bf_vsc(const double* mag, double* filt, int n_z, int n_x, void* stream);
+int launch_bf_h_list(const uint8_t* slot, int j, uint8_t* active, unsigned long long* fx, int n,
+                     void* stream);
+// the lines above the order statistic `rank` of filt: mask, magnitudes cleared, ascending list
+int launch_bf_nh_list(const double* filt, const uint8_t* lineok, int n, int rank, uint8_t* active,
+                      unsigned long long* fx, int* vis, int* n_vis, void* stream);
 int launch_bf_nh_mask(const double* filt, double thr, uint8_t* active, int n, void* stream);
 int launch_roi_sum(const DevGeom& g, int exact, int kind, const double* mag, const void* x,
                    int fp64, double* partial, double* out, void* stream);
@@ -394,6 +400,15 @@ int launch_rebuild_error(const void* y, void* e, const double* mu_old, const dou
                          int n_r, int n_t, int fp64, void* stream);
 int launch_prior_cost(const void* x, const DevFilter& f, int n_z, int n_x, int n_y,
                       double* partial, int n_blocks, int fp64, void* stream);
-int launch_reduce_stats(const double* in, int n_rows, int n_cols, double* out, void* stream);
+// err, count (device, or nullptr): copied behind the sums as three ints
+int launch_reduce_stats(const double* in, int n_rows, int n_cols, double* out, void* stream,
+                        const int* err = nullptr, const int* count = nullptr);
+// A sweep's or call's statistics as launch_reduce_stats leaves them, read back in one copy
+struct SweepResult {
+  double stat[kStatSlots];
+  int err;
+  int count[2];   // scheduled lines and classes (device schedules)
+  int pad;
+};
 
 }  // namespace mbir

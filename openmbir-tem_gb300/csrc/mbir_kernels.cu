@@ -345,7 +345,14 @@ __global__ void __launch_bounds__(256)
 
 // One warp per column (the sums are of 2^-32 multiples below 2^21 or counts: exact in any order)
 __global__ void reduce_rows_kernel(const double* __restrict__ in, int n_rows, int n_cols,
-                                   double* __restrict__ out) {
+                                   double* __restrict__ out, const int* __restrict__ err,
+                                   const int* __restrict__ count) {
+  if (threadIdx.x == 0 && err != nullptr) {
+    int* tail = reinterpret_cast<int*>(out + n_cols);
+    tail[0] = *err;
+    tail[1] = count != nullptr ? count[0] : 0;
+    tail[2] = count != nullptr ? count[1] : 0;
+  }
   const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (c >= n_cols) return;
   double s = 0.0;
@@ -542,9 +549,10 @@ int launch_prior_cost(const void* x, const DevFilter& f, int n_z, int n_x, int n
   }
   return ok_or(cudaGetLastError());
 }
-int launch_reduce_stats(const double* in, int n_rows, int n_cols, double* out, void* stream) {
+int launch_reduce_stats(const double* in, int n_rows, int n_cols, double* out, void* stream,
+                        const int* err, const int* count) {
   reduce_rows_kernel<<<1, 32 * n_cols, 0, static_cast<cudaStream_t>(stream)>>>(in, n_rows, n_cols,
-                                                                              out);
+                                                                              out, err, count);
   return ok_or(cudaGetLastError());
 }
 

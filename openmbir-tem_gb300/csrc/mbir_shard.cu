@@ -270,6 +270,7 @@ int Engine::bf_slab_end(const unsigned long long* mag) {
   if (mag)
     cudaMemcpyAsync(d_magfx_, mag, sizeof(unsigned long long) * nl, cudaMemcpyHostToDevice, s);
   slab_call_open_ = false;
+  bf_schedule_readback();
   int rc = bf_call_end();
   if (rc) return rc;
   if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "call end");
