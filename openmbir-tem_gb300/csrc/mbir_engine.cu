@@ -1062,7 +1062,7 @@ int Engine::forward_project() {
   const Geometry& g = g_;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   const size_t ns = static_cast<size_t>(g.n_t) * g.n_theta * n_rp_;
-  if (!stage_) cudaMemsetAsync(d_yest_, 0, rb_ * ns, s);
+  if (!stage_ || fp64_) cudaMemsetAsync(d_yest_, 0, rb_ * ns, s);
   std::vector<int32_t> rows(g.n_z);
   for (int i = 0; i < g.n_z; i++) rows[i] = i;
   cudaMemcpyAsync(d_rows_, rows.data(), sizeof(int) * g.n_z, cudaMemcpyHostToDevice, s);

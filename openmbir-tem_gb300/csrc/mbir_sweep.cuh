@@ -111,6 +111,41 @@ __device__ __forceinline__ uint32_t dynamic_smem_bytes() {
   return v;
 }
 
+// ---- thread-block clusters ----------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t v;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(v));
+  return v;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t v;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(v));
+  return v;
+}
+// every thread of every CTA of the cluster; what they wrote before is visible after
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;"
+               ::: "memory");
+}
+// p (in this CTA's shared memory) of CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void cluster_store(double* p, uint32_t rank, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(cluster_addr(p, rank)), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_store(float* p, uint32_t rank, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr(p, rank)), "f"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long cluster_load(const unsigned long long* p,
+                                                           uint32_t rank) {
+  unsigned long long v;
+  asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(cluster_addr(p, rank)) : "memory");
+  return v;
+}
+
 // ---- reductions within aligned groups of G lanes (all 32 lanes take part) -----------------
 template <int G, typename T>
 __device__ __forceinline__ T group_sum(T v) {
@@ -349,6 +384,7 @@ struct SliceCtx {
   const float4* acol;        // A-column table (level-scheduled sweeps) or nullptr
   const PriorConst<Real>* pc;  // prior and footprint constants (shared memory)
   const Real* qf;            // prior weights [27] (shared memory)
+  int ctas;                  // CTAs that share the slice (cluster sweeps), each with a cache
   bool coherent;             // neighbour planes read from the volume bypass L1 (other CTAs of
                              // the launch write them)
 };
@@ -384,10 +420,20 @@ __device__ __forceinline__ float f4_at(const float4& q, int k) {
   return k == 0 ? q.x : (k == 1 ? q.y : (k == 2 ? q.z : q.w));
 }
 
+// What other CTAs of the cluster write is read past L1 (CL)
+template <bool CL, typename T>
+__device__ __forceinline__ T shared_load(const T* p) {
+  if constexpr (CL)
+    return __ldcg(p);
+  else
+    return *p;
+}
+
 // With ACOL the voxel's A-column comes from the table (level-scheduled sweeps, FP32): the
 // same values the in-kernel computation gives, loaded first so that their latency overlaps
-// the neighbour loads.
-template <typename Real, int NB, int G, int VPL, bool BF, bool INLINE_ZS, bool ACOL = false>
+// the neighbour loads.  With CL the slice is shared by the CTAs of a cluster.
+template <typename Real, int NB, int G, int VPL, bool BF, bool INLINE_ZS, bool ACOL = false,
+          bool CL = false>
 __device__ __forceinline__ void group_step(const SliceCtx<Real>& c, int z, int x_req, int y,
                                            bool active, int lane, GroupAcc& acc) {
   using R2 = typename V2<Real>::type;
@@ -511,7 +557,8 @@ __device__ __forceinline__ void group_step(const SliceCtx<Real>& c, int z, int x
         Real* row = c.es + tr * c.ps + v * c.rs + jlo[i];
 #pragma unroll
         for (int b = 0; b < NB; ++b)
-          if (a[i][b] > Real(0)) row[b] += gain * (a[i][b] * hh * V);
+          if (a[i][b] > Real(0))
+            row[b] = shared_load<CL>(row + b) + gain * (a[i][b] * hh * V);
       }
     }
     return;
@@ -543,10 +590,10 @@ __device__ __forceinline__ void group_step(const SliceCtx<Real>& c, int z, int x
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         const bool ok = vok && a[i][b] > Real(0);
-        ev[i][b] = c.es[ok ? eidx[i] + b : 0];
+        ev[i][b] = shared_load<CL>(c.es + (ok ? eidx[i] + b : 0));
         if constexpr (BF) {
           wv[i][b] = __ldg(c.bw + (ok ? widx + b : 0));
-          sv[i][b] = c.bs[ok ? sidx + b : 0];
+          sv[i][b] = shared_load<CL>(c.bs + (ok ? sidx + b : 0));
         }
       }
     }
@@ -577,40 +624,54 @@ __device__ __forceinline__ void group_step(const SliceCtx<Real>& c, int z, int x
       }
     }
   } else {
+    // Several detector rows per slice (coarse levels): per view the entries of two rows in one
+    // batch of unconditional loads, as above.  Loaded one by one under their conditions, with the
+    // slice in HBM (which two rows of 512 bins at 61 views need), every entry was an L2 round
+    // trip of its own: 52k cycles per class of a bright-field call.
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
       const int v = gl + G * i;
       if (v >= g.n_theta || !live) continue;
       const R2 gw = c.sgw[v];
-      for (int tr = 0; tr < c.tcount; ++tr) {
-        const Real hh = c.hv[tr];
-        const Real* row = c.es + tr * c.ps + v * c.rs + jlo[i];
-        if constexpr (BF) {
-          const Real* wr = c.bw + tr * c.bw_ps + v * c.bw_rs + jlo[i];
-          const uint8_t* sr = c.bs + tr * c.bs_ps + v * c.bs_rs + jlo[i];
+      for (int tr0 = 0; tr0 < c.tcount; tr0 += 2) {
+        Real er[2][NB], wr[2][BN];
+        uint8_t sr[2][BN];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int tr = tr0 + k;
 #pragma unroll
           for (int b = 0; b < NB; ++b) {
-            if (a[i][b] > Real(0)) {
-              const Real e0 = row[b];
-              const Real w = __ldg(wr + b);
-              const Real pe = gw.x * a[i][b] * hh;
-              if (sr[b]) {
-                t2 += pe * pe * w;
-                t1 += e0 * pe * w;
-              } else {
-                const Real qc = c.bdt / (fabs(e0) * sqrt(w));
-                t2 += qc * (pe * pe * w);
-                t1 += qc * (e0 * pe * w);
-              }
+            const bool ok = tr < c.tcount && a[i][b] > Real(0);
+            er[k][b] = shared_load<CL>(c.es + (ok ? tr * c.ps + v * c.rs + jlo[i] + b : 0));
+            if constexpr (BF) {
+              wr[k][b] = __ldg(c.bw + (ok ? tr * c.bw_ps + v * c.bw_rs + jlo[i] + b : 0));
+              sr[k][b] = shared_load<CL>(c.bs + (ok ? tr * c.bs_ps + v * c.bs_rs + jlo[i] + b : 0));
             }
           }
-        } else {
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          if (tr0 + k >= c.tcount) continue;
+          const Real hh = c.hv[tr0 + k];
 #pragma unroll
           for (int b = 0; b < NB; ++b) {
             if (a[i][b] > Real(0)) {
+              const Real e0 = er[k][b];
               const Real pe = gw.x * a[i][b] * hh;
-              t2 += pe * pe * gw.y;
-              t1 += row[b] * pe * gw.y;
+              if constexpr (BF) {
+                const Real w = wr[k][b];
+                if (sr[k][b]) {
+                  t2 += pe * pe * w;
+                  t1 += e0 * pe * w;
+                } else {
+                  const Real qc = c.bdt / (fabs(e0) * sqrt(w));
+                  t2 += qc * (pe * pe * w);
+                  t1 += qc * (e0 * pe * w);
+                }
+              } else {
+                t2 += pe * pe * gw.y;
+                t1 += e0 * pe * gw.y;
+              }
             }
           }
         }
@@ -668,31 +729,50 @@ __device__ __forceinline__ void group_step(const SliceCtx<Real>& c, int z, int x
         const int v = gl + G * i;
         if (v >= g.n_theta) continue;
         const Real gain = c.sgw[v].x;
-        for (int tr = 0; tr < c.tcount; ++tr) {
-          const Real hh = c.hv[tr];
-          Real* row = c.es + tr * c.ps + v * c.rs + jlo[i];
-          if constexpr (BF) {
-            const Real* wr = c.bw + tr * c.bw_ps + v * c.bw_rs + jlo[i];
-            uint8_t* sr = c.bs + tr * c.bs_ps + v * c.bs_rs + jlo[i];
+        for (int tr0 = 0; tr0 < c.tcount; tr0 += 2) {
+          Real er[2][NB], wr[2][BN];
+          uint8_t sr[2][BN];
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int tr = tr0 + k;
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+              const bool ok = tr < c.tcount && a[i][b] > Real(0);
+              er[k][b] = shared_load<CL>(c.es + (ok ? tr * c.ps + v * c.rs + jlo[i] + b : 0));
+              if constexpr (BF) {
+                wr[k][b] = __ldg(c.bw + (ok ? tr * c.bw_ps + v * c.bw_rs + jlo[i] + b : 0));
+                sr[k][b] =
+                    shared_load<CL>(c.bs + (ok ? tr * c.bs_ps + v * c.bs_rs + jlo[i] + b : 0));
+              }
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int tr = tr0 + k;
+            if (tr >= c.tcount) continue;
+            const Real hh = c.hv[tr];
+            Real* row = c.es + tr * c.ps + v * c.rs + jlo[i];
 #pragma unroll
             for (int b = 0; b < NB; ++b)
               if (a[i][b] > Real(0)) {
-                const Real ne = row[b] - gain * (a[i][b] * hh * dlt);
+                const Real ne = er[k][b] - gain * (a[i][b] * hh * dlt);
                 row[b] = ne;
-                sr[b] = bragg_selected<Real>(ne, __ldg(wr + b), c.bt);
+                if constexpr (BF) {  // (the selector seldom changes)
+                  const uint8_t on = bragg_selected<Real>(ne, wr[k][b], c.bt);
+                  if (on != sr[k][b]) c.bs[tr * c.bs_ps + v * c.bs_rs + jlo[i] + b] = on;
+                }
               }
-          } else {
-#pragma unroll
-            for (int b = 0; b < NB; ++b)
-              if (a[i][b] > Real(0)) row[b] -= gain * (a[i][b] * hh * dlt);
           }
         }
       }
     }
   }
+  if constexpr (CL) {
+    if (gl < c.ctas) cluster_store(c.cache + 4 * g.n_x + x, gl, nv);
+  }
   if (gl == 0) {
     c.vol[vidx] = nv;
-    if (c.cache) c.cache[4 * g.n_x + x] = nv;
+    if (!CL && c.cache) c.cache[4 * g.n_x + x] = nv;
     if (x >= g.roi_x0 && x <= g.roi_x1 && z >= g.roi_z0 && z <= g.roi_z1) {
       acc.v[0] += fix32<Real>(dlt);
       acc.v[1] += fix32<Real>(V);
@@ -782,7 +862,10 @@ __host__ __device__ inline SmemLayout smem_layout(int n_theta, int n_x, int n_rs
 // slices); `coherent` makes neighbour-row loads bypass L1 (needed when other CTAs of the same
 // launch write neighbouring slices).  Writes the slice's four statistics to stat_out when it
 // is not null.  Returns false when a bounded wait gave up (A.err is set).
-template <typename Real, int NB, int G, int VPL, bool STAGE, bool BF>
+// CL: the CTAs of a cluster share the slice (in HBM).  Each walks the rows with its own cache and
+// lists and updates every ctas-th voxel of a step; a voxel's new value goes to every cache, and
+// the step ends with a cluster barrier.
+template <typename Real, int NB, int G, int VPL, bool STAGE, bool BF, bool CL = false>
 __device__ __forceinline__ bool run_slice(const SweepArgs& A, int y, unsigned char* smem,
                                           uint32_t& phase, bool coherent, double* stat_out) {
   using R2 = typename V2<Real>::type;
@@ -792,6 +875,9 @@ __device__ __forceinline__ bool run_slice(const SweepArgs& A, int y, unsigned ch
   constexpr int GPW = 32 / G;  // voxel groups per warp
   const int group = warp * GPW + (lane / G);
   const int n_groups = (nthreads / 32) * GPW;
+  static_assert(!CL || !STAGE, "a shared slice lies in HBM");
+  const int ctas = CL ? static_cast<int>(cluster_size()) : 1;
+  const int rank = CL ? static_cast<int>(cluster_rank()) : 0;
   const int tcount = A.tab.t_count[y], tfirst = A.tab.t_first[y];
   const int n_sp = BF ? A.bfa.n_sp : 0;
   const bool sched_layout = BF && std::is_same<Real, float>::value && A.sched_lines != nullptr &&
@@ -913,6 +999,7 @@ __device__ __forceinline__ bool run_slice(const SweepArgs& A, int y, unsigned ch
   c.bt = c.bdt = Real(0);
   c.acol = nullptr;
   c.coherent = coherent;
+  c.ctas = ctas;
   c.pc = &s_pc;
   c.qf = s_qf;
   if (BF) {
@@ -1149,14 +1236,19 @@ __device__ __forceinline__ bool run_slice(const SweepArgs& A, int y, unsigned ch
     }
     __syncthreads();
     const int n_steps = static_cast<int>(ctl[0]);
+    if constexpr (CL) cluster_sync();  // every CTA's cache holds the row before values go there
     for (int st = 0; st < n_steps; ++st) {
       const int b = gofs[st], n = gofs[st + 1] - b;
-      for (int b0 = 0; b0 < n; b0 += n_groups) {
-        const int i = b0 + group;
+      for (int b0 = 0; b0 < n; b0 += n_groups * ctas) {
+        const int i = b0 + group * ctas + rank;
         const bool act = i < n;
-        group_step<Real, NB, G, VPL, BF, false>(c, z, act ? flat[b + i] : 0, y, act, lane, acc);
+        group_step<Real, NB, G, VPL, BF, false, false, CL>(c, z, act ? flat[b + i] : 0, y, act,
+                                                           lane, acc);
       }
-      __syncthreads();
+      if constexpr (CL)
+        cluster_sync();
+      else
+        __syncthreads();
     }
   }
 
@@ -1185,8 +1277,22 @@ __device__ __forceinline__ bool run_slice(const SweepArgs& A, int y, unsigned ch
     if (tid < kStatSlots) {
       unsigned long long t = 0;
       for (int w = 0; w < n_groups; ++w) t += sstat[w * kStatSlots + tid];
+      if constexpr (CL) sstat[tid] = t;  // (this column's first slot, read above)
       if (tid == 2) t += ctl[2];
-      stat_out[tid] = tid < 2 ? static_cast<double>(t) / kFixScale : static_cast<double>(t);
+      if constexpr (!CL)
+        stat_out[tid] = tid < 2 ? static_cast<double>(t) / kFixScale : static_cast<double>(t);
+      else
+        sstat[kStatSlots + tid] = t;
+    }
+    if constexpr (CL) {
+      // every CTA's updates; the voxels skipped with their row are the same in each (ctl[2])
+      cluster_sync();
+      if (rank == 0 && tid < kStatSlots) {
+        unsigned long long t = sstat[kStatSlots + tid];
+        for (int r = 1; r < ctas; ++r) t += cluster_load(sstat + tid, r);
+        stat_out[tid] = tid < 2 ? static_cast<double>(t) / kFixScale : static_cast<double>(t);
+      }
+      cluster_sync();  // until here no CTA's shared memory goes away
     }
   }
   __syncthreads();
@@ -1213,6 +1319,21 @@ __global__ void __launch_bounds__(kWarps * 32, 1) sweep_kernel(const __grid_cons
   run_slice<Real, NB, G, VPL, STAGE, BF>(
       A, y, smem, phase, false,
       A.stats != nullptr ? A.stats + static_cast<size_t>(blockIdx.x) * kStatSlots : nullptr);
+}
+
+// The slices of one y-colour, each by a cluster of CTAs (the FP64 engine's small volumes)
+template <typename Real, int NB, int G, int VPL, bool BF>
+__global__ void __launch_bounds__(kWarps * 32, 1)
+    cluster_sweep_kernel(const __grid_constant__ SweepArgs A) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int slice = static_cast<int>(blockIdx.x / cluster_size());
+  const int y = (A.y_end > 0 ? A.y_first : A.colour) + 2 * slice;
+  if (y >= (A.y_end > 0 ? A.y_end : A.g.n_y)) return;
+  init_slice_barrier(smem);
+  uint32_t phase = 0;
+  run_slice<Real, NB, G, VPL, false, BF, true>(
+      A, y, smem, phase, true,
+      A.stats != nullptr ? A.stats + static_cast<size_t>(slice) * kStatSlots : nullptr);
 }
 
 // One slice of a batched series with its staging.
@@ -1462,6 +1583,35 @@ int launch_slices(const SweepArgs& a, size_t smem, int threads, cudaStream_t s) 
   }
   k<<<a.n_slices, threads, smem, s>>>(a);
   return ok_or(cudaGetLastError());
+}
+
+// The launch with `ctas` CTAs per slice; 1 when the device does not hold that many clusters at once
+template <auto k>
+int launch_clusters(const SweepArgs& a, size_t smem, int ctas, cudaStream_t s, bool& launched) {
+  launched = false;
+  static const int lim = dyn_smem_limit(k);
+  if (smem > static_cast<size_t>(lim)) return 0;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess)
+    return -3;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(ctas);
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(a.n_slices * ctas));
+  cfg.blockDim = dim3(kWarps * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int fit = 0;
+  if (cudaOccupancyMaxActiveClusters(&fit, k, &cfg) != cudaSuccess || fit < a.n_slices) {
+    cudaGetLastError();
+    return 0;
+  }
+  launched = true;
+  return ok_or(cudaLaunchKernelEx(&cfg, k, a));
 }
 
 template <typename Real, int NB, int G, int VPL, bool STAGE, bool BF>
