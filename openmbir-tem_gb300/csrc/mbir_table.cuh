@@ -103,6 +103,57 @@ __device__ __forceinline__ float qggmrf_coef_tab(const PriorF& q, float d0) {
   return d0 == 0.f ? q.P / (q.sp * q.c) : r;
 }
 
+// The three weights at row[j..j+2], from 16-byte loads: rows in memory are whole 16 bytes, so the
+// values lie in two windows of four, each read only when one of its values has a footprint value
+// `a` (others are undefined).  A gather's lanes read neighbouring values of 32 different rows, and
+// L1 takes about one row per clock, which bounds the classes of a bright-field call whose slices
+// lie in HBM: 1.5 loads per view instead of 3 (and 1.25 instead of 3 for the selector), with the
+// unchanged selector bytes not written, took six calls of the 1024 x 512 x 256 volume at 121 views
+// from 158 to 115 ms.  Windows for the error as well: 117 ms; for weights of slices in shared
+// memory 17.1 -> 19.8 ms, for HAADF errors 40.8 -> 50, for the coarse level's two rows 40 -> 60:
+// there latency and instructions count, not the number of loads.
+template <int NB>
+__device__ __forceinline__ void gather_row(const float* row, int j, const float (&a)[NB],
+                                           float (&out)[NB]) {
+  static_assert(NB == 3, "two windows of four");
+  const int k = j & ~3, off = j & 3;
+  bool p0 = false, p1 = false;
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    p0 |= a[b] > 0.f && off + b < 4;
+    p1 |= a[b] > 0.f && off + b >= 4;
+  }
+  const float4* q = reinterpret_cast<const float4*>(row + k);
+  float4 w0 = make_float4(0.f, 0.f, 0.f, 0.f), w1 = w0;
+  if (p0) w0 = __ldg(q);
+  if (p1) w1 = __ldg(q + 1);
+  const float v[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+  float u[NB + 1];
+#pragma unroll
+  for (int b = 0; b <= NB; ++b) u[b] = (off & 2) ? v[b + 2] : v[b];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) out[b] = (off & 1) ? u[b + 1] : u[b];
+}
+// The same for selector bytes (rows of whole 8 bytes, two windows of eight)
+template <int NB>
+__device__ __forceinline__ void gather_row(const uint8_t* row, int j, const float (&a)[NB],
+                                           unsigned (&out)[NB]) {
+  const int k = j & ~7, off = j & 7;
+  bool p0 = false, p1 = false;
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    p0 |= a[b] > 0.f && off + b < 8;
+    p1 |= a[b] > 0.f && off + b >= 8;
+  }
+  const unsigned long long* q = reinterpret_cast<const unsigned long long*>(row + k);
+  unsigned long long w0 = 0ull, w1 = 0ull;
+  if (p0) w0 = q[0];
+  if (p1) w1 = q[1];
+  const unsigned long long w = off ? (w0 >> (8 * off)) | (w1 << (64 - 8 * off)) : w0;
+#pragma unroll
+  for (int b = 0; b < NB; ++b) out[b] = static_cast<unsigned>(w >> (8 * b)) & 0xffu;
+}
+
 // One updated voxel in the sweep's statistics, its line's magnitude for bright field
 template <bool BF>
 __device__ __forceinline__ void count_update(const SweepArgs& A, unsigned long long* mag_fx, int z,
@@ -175,31 +226,31 @@ __device__ __forceinline__ void table_step(const SweepArgs& A, const TabCtx<G, V
   }
 
   // footprint entries, all in flight together
+  constexpr bool kWide = BF && !STAGE;  // weights and selector by windows (gather_row)
   float ev[VPL][NB];
   float wv[BF ? VPL : 1][NB];
   unsigned sv[BF ? VPL : 1][NB];
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
     const int j = __float_as_int(aq[i].x);
+    const float a[NB] = {aq[i].y, aq[i].z, aq[i].w};
     const float* er = c.es + (c.eoff[i] + j);
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
-      const bool p = f4_at(aq[i], b + 1) > 0.f;
-      if constexpr (STAGE) {
-        ev[i][b] = er[b];
-      } else {
-        ev[i][b] = 0.f;
-        if (p) ev[i][b] = er[b];
-      }
-      if constexpr (BF) {
+      ev[i][b] = 0.f;
+      if (STAGE || a[b] > 0.f) ev[i][b] = er[b];
+    }
+    if constexpr (kWide) {
+      gather_row<NB>(c.bw + c.woff[i], j, a, wv[i]);
+      gather_row<NB>(c.bs + c.soff[i], j, a, sv[i]);
+    } else if constexpr (BF) {
+      const float* wr = c.bw + (c.woff[i] + j);
+      const uint8_t* sr = c.bs + (c.soff[i] + j);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
         wv[i][b] = 0.f;
-        if (p) wv[i][b] = __ldg(c.bw + (c.woff[i] + j) + b);
-        if constexpr (STAGE) {
-          sv[i][b] = c.bs[c.soff[i] + j + b];
-        } else {
-          sv[i][b] = 1;
-          if (p) sv[i][b] = c.bs[c.soff[i] + j + b];
-        }
+        if (a[b] > 0.f) wv[i][b] = __ldg(wr + b);
+        sv[i][b] = sr[b];
       }
     }
   }
@@ -292,8 +343,13 @@ __device__ __forceinline__ void table_step(const SweepArgs& A, const TabCtx<G, V
         const float ne = ev[i][b] - c.gx[i] * (a * c.hh * dlt);
         if (a > 0.f) {
           er[b] = ne;
-          if constexpr (BF)
-            c.bs[c.soff[i] + j + b] = bragg_selected<float>(ne, wv[i][b], c.bt);
+          if constexpr (BF) {
+            // the selector seldom changes: in HBM its byte is then not written (a fifth of the
+            // call's time at 1024 bins and 121 views); in shared memory the test costs more than
+            // the store (19.0 against 17.1 ms of sweep kernels per equivalent iteration)
+            const unsigned on = bragg_selected<float>(ne, wv[i][b], c.bt);
+            if (STAGE || on != sv[i][b]) c.bs[c.soff[i] + j + b] = static_cast<uint8_t>(on);
+          }
         }
       }
     }
