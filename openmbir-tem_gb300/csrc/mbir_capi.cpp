@@ -378,8 +378,9 @@ int32_t mbir_run_multires(const mbir_params* p, const float* counts, const float
   const mbir_params top = with_float_params(*p);
   p = &top;
   const int levels = p->num_resolutions > 0 ? p->num_resolutions : 1;
-  std::vector<double> prev;
+  mbir::HostVolume prev;
   int pdims[3] = {0, 0, 0};
+  bool out_filled = false;
   std::vector<double> g(n_theta), o(n_theta), v(n_theta);
   bool have_nuis = false;
   try {
@@ -400,23 +401,33 @@ int32_t mbir_run_multires(const mbir_params* p, const float* counts, const float
       if (i > 0) {
         // 2x voxel replication of the previous level (InterpFlag = 1), in FP64 as the
         // reference reads ReconstructedObject.bin
-        std::vector<double> up(static_cast<size_t>(d[0]) * d[1] * d[2], 0.0);
-        const int ze = d[0] / 2, xe = d[1] / 2, ye = d[2] / 2;
-        for (int y = 0; y < ye && y < pdims[2]; y++)
-          for (int x = 0; x < xe && x < pdims[1]; x++)
-            for (int z = 0; z < ze && z < pdims[0]; z++) {
-              const double b = prev[(static_cast<size_t>(z) * pdims[1] + x) * pdims[2] + y];
-              for (int a = 0; a < 2; a++)
-                for (int c = 0; c < 2; c++)
-                  for (int r = 0; r < 2; r++)
-                    up[(static_cast<size_t>(2 * z + a) * d[1] + 2 * x + c) * d[2] + 2 * y + r] = b;
+        mbir::HostVolume up(static_cast<size_t>(d[0]) * d[1] * d[2]);
+        const int ze = std::min(d[0] / 2, pdims[0]), xe = std::min(d[1] / 2, pdims[1]),
+                  ye = std::min(d[2] / 2, pdims[2]);
+        mbir::host_parallel(d[0], [&](int z_begin, int z_end) {
+          for (int z = z_begin; z < z_end; z++)
+            for (int x = 0; x < d[1]; x++) {
+              double* row = up.data() + (static_cast<size_t>(z) * d[1] + x) * d[2];
+              int y = 0;
+              if (z < 2 * ze && x < 2 * xe) {
+                const double* from =
+                    prev.data() + (static_cast<size_t>(z / 2) * pdims[1] + x / 2) * pdims[2];
+                for (; y < 2 * ye; y++) row[y] = from[y / 2];
+              }
+              for (; y < d[2]; y++) row[y] = 0.0;
             }
-        if ((rc = eng.set_initial_volume_f64(up.data(), static_cast<int64_t>(up.size()))))
-          return rc;
+        });
+        if ((rc = eng.adopt_initial_volume(std::move(up)))) return rc;
       }
       if ((rc = eng.run())) return rc;
-      prev.assign(static_cast<size_t>(d[0]) * d[1] * d[2], 0.0);
-      if ((rc = eng.get_volume_f64(prev.data(), static_cast<int64_t>(prev.size())))) return rc;
+      const size_t nv = static_cast<size_t>(d[0]) * d[1] * d[2];
+      if (i + 1 < levels) {
+        prev.resize(nv);
+        if ((rc = eng.get_volume_f64(prev.data(), static_cast<int64_t>(nv)))) return rc;
+      } else if (out && n >= static_cast<int64_t>(nv)) {
+        if ((rc = eng.get_volume(out, n))) return rc;
+        out_filled = true;
+      }
       pdims[0] = d[0];
       pdims[1] = d[1];
       pdims[2] = d[2];
@@ -432,10 +443,7 @@ int32_t mbir_run_multires(const mbir_params* p, const float* counts, const float
     dims_out[1] = pdims[1];
     dims_out[2] = pdims[2];
   }
-  if (out) {
-    if (n < static_cast<int64_t>(nv)) return MBIR_EINVAL;
-    for (size_t i = 0; i < nv; i++) out[i] = static_cast<float>(prev[i]);
-  }
+  if (out && !out_filled && n < static_cast<int64_t>(nv)) return MBIR_EINVAL;
   return MBIR_OK;
 }
 

@@ -293,6 +293,15 @@ int Engine::set_initial_volume_t(const T* vol, int64_t n) {
   return MBIR_OK;
 }
 
+int Engine::adopt_initial_volume(HostVolume&& vol) {
+  if (p_.interpolate_initial_recon)
+    return set_initial_volume_f64(vol.data(), static_cast<int64_t>(vol.size()));
+  if (vol.empty()) return fail(MBIR_EINVAL, "set_initial_volume: bad arguments");
+  init_vol_ = std::move(vol);
+  host_ready_ = false;
+  return MBIR_OK;
+}
+
 int Engine::set_initial_volume(const float* vol, int64_t n) {
   return set_initial_volume_t(vol, n);
 }
@@ -517,37 +526,38 @@ int Engine::build_tables() {
 int Engine::compute_stride() {
   const Geometry& g = g_;
   const double d = g.delta_xz / g.delta_r, eps = 1e-4;
-  int S = 2;
-  for (; S < g.n_x; ++S) {
-    // any conflict at this stride, searched over rows in parallel (a yes/no answer)
-    std::atomic<bool> found{false};
-    host_parallel(g.n_z, [&](int z_begin, int z_end) {
-      bool conflict = false;
-      for (int v = 0; v < g.n_theta && !conflict; ++v) {
-        const double bxv = g.delta_xz * tab_.cosv[v] / g.delta_r;
-        const double bzv = g.delta_xz * tab_.sinv[v] / g.delta_r;
-        const double u0 = ((g.x0 + 0.5 * g.delta_xz) * tab_.cosv[v] -
-                           (g.z0 + 0.5 * g.delta_xz) * tab_.sinv[v] - g.R0) /
-                          g.delta_r;
-        if (found.load(std::memory_order_relaxed)) break;
-        for (int z = z_begin; z < z_end && !conflict; ++z) {
-          for (int x = 0; x + S < g.n_x; ++x) {
-            const double ua = u0 + x * bxv - z * bzv, ub = ua + S * bxv;
-            double alo = std::floor(ua - d - eps), ahi = std::floor(ua + d + eps);
-            double blo = std::floor(ub - d - eps), bhi = std::floor(ub + d + eps);
-            alo = std::max(alo, 0.0);
-            blo = std::max(blo, 0.0);
-            ahi = std::min(ahi, (double)g.n_r - 1);
-            bhi = std::min(bhi, (double)g.n_r - 1);
-            if (alo > ahi || blo > bhi) continue;
-            if (!(ahi < blo || bhi < alo)) {
-              conflict = true;
-              break;
-            }
-          }
+  // two voxels of rows [z_begin, z_end) at distance S share a bin at some view
+  auto conflict = [&](int S, int z_begin, int z_end, const std::atomic<bool>& found) {
+    for (int v = 0; v < g.n_theta; ++v) {
+      const double bxv = g.delta_xz * tab_.cosv[v] / g.delta_r;
+      const double bzv = g.delta_xz * tab_.sinv[v] / g.delta_r;
+      const double u0 = ((g.x0 + 0.5 * g.delta_xz) * tab_.cosv[v] -
+                         (g.z0 + 0.5 * g.delta_xz) * tab_.sinv[v] - g.R0) /
+                        g.delta_r;
+      if (found.load(std::memory_order_relaxed)) return false;
+      for (int z = z_begin; z < z_end; ++z) {
+        for (int x = 0; x + S < g.n_x; ++x) {
+          const double ua = u0 + x * bxv - z * bzv, ub = ua + S * bxv;
+          double alo = std::floor(ua - d - eps), ahi = std::floor(ua + d + eps);
+          double blo = std::floor(ub - d - eps), bhi = std::floor(ub + d + eps);
+          alo = std::max(alo, 0.0);
+          blo = std::max(blo, 0.0);
+          ahi = std::min(ahi, (double)g.n_r - 1);
+          bhi = std::min(bhi, (double)g.n_r - 1);
+          if (alo > ahi || blo > bhi) continue;
+          if (!(ahi < blo || bhi < alo)) return true;
         }
       }
-      if (conflict) found.store(true);
+    }
+    return false;
+  };
+  int S = 2;
+  for (; S < g.n_x; ++S) {
+    // a stride that is too small conflicts in every row: one row tells without the threads
+    std::atomic<bool> found{false};
+    if (conflict(S, g.n_z / 2, g.n_z / 2 + 1, found)) continue;
+    host_parallel(g.n_z, [&](int z_begin, int z_end) {
+      if (conflict(S, z_begin, z_end, found)) found.store(true);
     });
     if (!found.load()) break;
   }
@@ -868,38 +878,51 @@ int Engine::prepare() {
 
   // initial volume (InitialReconstructionInitializer::initializeData, :74-90)
   const size_t nv = static_cast<size_t>(g.n_z) * g.n_x * g.n_y;
-  std::vector<double> vol(nv);
-  if (!init_vol_.empty()) {
-    if (init_vol_.size() != nv) return fail(MBIR_EINVAL, "initial volume size does not match");
-    vol = init_vol_;
-  } else {
-    std::fill(vol.begin(), vol.end(), fp64_ ? p_.default_recon_value
-                                            : static_cast<double>(static_cast<float>(
-                                                  p_.default_recon_value)));
-  }
-  for (int z = 0; z < g.n_z; z++)
-    for (int x = 0; x < g.n_x; x++)
-      if (!tab_.line_nonempty[static_cast<size_t>(z) * g.n_x + x])
-        for (int y = 0; y < g.n_y; y++) vol[(static_cast<size_t>(z) * g.n_x + x) * g.n_y + y] = 0.0;
-  if (fp64_) {
-    // the doubles as given (an FP64 engine starts exactly where the reference starts)
-    double* tmp = nullptr;
-    if (cudaMalloc(&tmp, sizeof(double) * nv) != cudaSuccess) {
-      cudaGetLastError();
-      return fail(MBIR_ENOMEM, "volume upload: device allocation failed");
-    }
-    cudaMemcpyAsync(tmp, vol.data(), sizeof(double) * nv, cudaMemcpyHostToDevice, s);
-    rc = launch_vol64_to_dev(tmp, d_x_, g.n_z, g.n_x, g.n_y, fp64_, s);
-    const bool ok = cudaStreamSynchronize(s) == cudaSuccess;
-    cudaFree(tmp);
-    if (rc) return cuda_check(rc, "volume upload");
-    if (!ok) return cuda_check(MBIR_EDEVICE, "prepare sync");
-  } else {
-    std::vector<float> vf(vol.begin(), vol.end());
-    cudaMemcpyAsync(d_stage_, vf.data(), sizeof(float) * nv, cudaMemcpyHostToDevice, s);
-    if ((rc = launch_vol_to_dev(d_stage_, d_x_, g.n_z, g.n_x, g.n_y, fp64_, s)))
-      return cuda_check(rc, "volume upload");
+  if (init_vol_.empty()) {
+    const double value = fp64_ ? p_.default_recon_value
+                               : static_cast<double>(static_cast<float>(p_.default_recon_value));
+    if ((rc = launch_fill_volume(d_x_, value, d_lineok_, g.n_z * g.n_x, g.n_y, fp64_, s)))
+      return cuda_check(rc, "volume fill");
     if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "prepare sync");
+  } else {
+    if (init_vol_.size() != nv) return fail(MBIR_EINVAL, "initial volume size does not match");
+    // lines without an A-column start at 0
+    auto masked = [&](auto* to) {
+      using T = std::remove_pointer_t<decltype(to)>;
+      host_parallel(g.n_z * g.n_x, [&](int l_begin, int l_end) {
+        for (int l = l_begin; l < l_end; l++) {
+          const double* from = init_vol_.data() + static_cast<size_t>(l) * g.n_y;
+          T* row = to + static_cast<size_t>(l) * g.n_y;
+          if (tab_.line_nonempty[l])
+            for (int y = 0; y < g.n_y; y++) row[y] = static_cast<T>(from[y]);
+          else
+            std::fill(row, row + g.n_y, T(0));
+        }
+      });
+    };
+    if (fp64_) {
+      // the doubles as given (an FP64 engine starts exactly where the reference starts)
+      std::unique_ptr<double[]> vol(new double[nv]);
+      masked(vol.get());
+      double* tmp = nullptr;
+      if (cudaMalloc(&tmp, sizeof(double) * nv) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(MBIR_ENOMEM, "volume upload: device allocation failed");
+      }
+      cudaMemcpyAsync(tmp, vol.get(), sizeof(double) * nv, cudaMemcpyHostToDevice, s);
+      rc = launch_vol64_to_dev(tmp, d_x_, g.n_z, g.n_x, g.n_y, fp64_, s);
+      const bool ok = cudaStreamSynchronize(s) == cudaSuccess;
+      cudaFree(tmp);
+      if (rc) return cuda_check(rc, "volume upload");
+      if (!ok) return cuda_check(MBIR_EDEVICE, "prepare sync");
+    } else {
+      std::unique_ptr<float[]> vol(new float[nv]);
+      masked(vol.get());
+      cudaMemcpyAsync(d_stage_, vol.get(), sizeof(float) * nv, cudaMemcpyHostToDevice, s);
+      if ((rc = launch_vol_to_dev(d_stage_, d_x_, g.n_z, g.n_x, g.n_y, fp64_, s)))
+        return cuda_check(rc, "volume upload");
+      if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "prepare sync");
+    }
   }
 
   // device geometry + prior constants
@@ -1579,17 +1602,29 @@ int Engine::get_volume_f64(double* out, int64_t n) {
   const size_t nv = static_cast<size_t>(g.n_z) * g.n_x * g.n_y;
   if (!out || n < static_cast<int64_t>(nv)) return fail(MBIR_EINVAL, "get_volume: buffer too small");
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  std::vector<unsigned char> raw(nv * rb_);
-  cudaMemcpyAsync(raw.data(), d_x_, raw.size(), cudaMemcpyDeviceToHost, s);
+  if (!fp64_) {  // transposed on the device, widened here
+    std::unique_ptr<float[]> vol(new float[nv]);
+    const int rc = launch_vol_to_host(d_x_, d_stage_, g.n_z, g.n_x, g.n_y, fp64_, s);
+    if (rc) return cuda_check(rc, "volume read-out");
+    cudaMemcpyAsync(vol.get(), d_stage_, sizeof(float) * nv, cudaMemcpyDeviceToHost, s);
+    if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "volume read-out");
+    host_parallel(g.n_z, [&](int z_begin, int z_end) {
+      const size_t b = static_cast<size_t>(z_begin) * g.n_x * g.n_y;
+      const size_t e = static_cast<size_t>(z_end) * g.n_x * g.n_y;
+      for (size_t i = b; i < e; i++) out[i] = static_cast<double>(vol[i]);
+    });
+    return MBIR_OK;
+  }
+  std::unique_ptr<double[]> raw(new double[nv]);
+  cudaMemcpyAsync(raw.get(), d_x_, sizeof(double) * nv, cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "volume read-out");
-  for (int y = 0; y < g.n_y; y++)
-    for (int z = 0; z < g.n_z; z++)
-      for (int x = 0; x < g.n_x; x++) {
-        const size_t i = (static_cast<size_t>(y) * g.n_z + z) * g.n_x + x;
-        const double v = fp64_ ? reinterpret_cast<const double*>(raw.data())[i]
-                               : static_cast<double>(reinterpret_cast<const float*>(raw.data())[i]);
-        out[(static_cast<size_t>(z) * g.n_x + x) * g.n_y + y] = v;
-      }
+  host_parallel(g.n_z, [&](int z_begin, int z_end) {
+    for (int z = z_begin; z < z_end; z++)
+      for (int y = 0; y < g.n_y; y++)
+        for (int x = 0; x < g.n_x; x++)
+          out[(static_cast<size_t>(z) * g.n_x + x) * g.n_y + y] =
+              raw[(static_cast<size_t>(y) * g.n_z + z) * g.n_x + x];
+  });
   return MBIR_OK;
 }
 

@@ -76,6 +76,9 @@ class MT19937 {
 // visit order of UpdateYSlice::execute (HAADF_ReconstructionEngine_UpdateVoxels.cpp:151-241)
 void reference_visit_order(uint32_t seed, int n_z, int n_x, std::vector<int32_t>& out);
 
+// A host volume [z][x][y] whose values are all written by whoever sizes it
+using HostVolume = std::vector<double, UninitAlloc<double>>;
+
 class Engine {
  public:
   explicit Engine(const mbir_params& p);
@@ -85,6 +88,7 @@ class Engine {
                    double delta_r, double delta_t);
   int load_mrc(const char* path);
   int set_initial_volume_f64(const double* vol, int64_t n);
+  int adopt_initial_volume(HostVolume&& vol);  // set_initial_volume_f64 without the copy
   // HAADF: after every inner iteration the volume as <dir>/<outer>_<inner>_ReconstructedVolume.rec
   int set_intermediate_dir(const char* dir);
   int set_observer(mbir_observer_fn fn, void* user);
@@ -248,7 +252,7 @@ class Engine {
   std::vector<double> resume_gain_, resume_offset_, resume_var_;
   void* observer_user_ = nullptr;
   std::vector<double> tilts_;     // degrees
-  std::vector<double> init_vol_;  // optional [z][x][y]
+  HostVolume init_vol_;           // optional [z][x][y]
   std::vector<double> user_gain_, user_offset_, user_var_;
 
   Geometry g_;

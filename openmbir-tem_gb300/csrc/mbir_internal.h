@@ -375,6 +375,9 @@ int launch_sino_to_dev(const float* host_layout, void* dev_layout, int n_theta, 
                        int n_t, int fp64, void* stream);
 int launch_sino_to_host(const void* dev_layout, float* host_layout, int n_theta, int n_r,
                         int n_rp, int n_t, int fp64, void* stream);
+// every voxel of a line to `value`, 0 where lineok is 0
+int launch_fill_volume(void* yzx, double value, const uint8_t* lineok, int n_lines, int n_y,
+                       int fp64, void* stream);
 int launch_vol_to_dev(const float* zxy, void* yzx, int n_z, int n_x, int n_y, int fp64,
                       void* stream);
 // the same from an FP64 volume in device memory ([z][x][y] doubles)

@@ -60,6 +60,15 @@ __global__ void sino_to_host_kernel(const Real* __restrict__ d, float* __restric
   }
 }
 template <typename Real>
+__global__ void fill_volume_kernel(Real* __restrict__ x, Real value,
+                                   const uint8_t* __restrict__ lineok, int n_lines, int n_y) {
+  for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < n_lines; l += gridDim.x * blockDim.x) {
+    const Real v = lineok[l] ? value : Real(0);
+    for (int y = blockIdx.y; y < n_y; y += gridDim.y)
+      x[static_cast<size_t>(y) * n_lines + l] = v;
+  }
+}
+template <typename Real>
 __global__ void vol_to_dev_kernel(const float* __restrict__ zxy, Real* __restrict__ yzx, int n_z,
                                   int n_x, int n_y) {
   const size_t total = static_cast<size_t>(n_z) * n_x * n_y;
@@ -429,6 +438,17 @@ int launch_sino_to_host(const void* d, float* h, int n_theta, int n_r, int n_rp,
   else
     sino_to_host_kernel<float><<<grid_for(n, 256), 256, 0, s>>>(RP<float>(d), h, n_theta, n_r,
                                                                  n_rp, n_t);
+  return ok_or(cudaGetLastError());
+}
+int launch_fill_volume(void* yzx, double value, const uint8_t* lineok, int n_lines, int n_y,
+                       int fp64, void* stream) {
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const dim3 grid(std::max(1, std::min((n_lines + 255) / 256, 1024)), std::max(1, std::min(n_y, 32)));
+  if (fp64)
+    fill_volume_kernel<double><<<grid, 256, 0, s>>>(RP<double>(yzx), value, lineok, n_lines, n_y);
+  else
+    fill_volume_kernel<float><<<grid, 256, 0, s>>>(RP<float>(yzx), static_cast<float>(value), lineok,
+                                                   n_lines, n_y);
   return ok_or(cudaGetLastError());
 }
 int launch_vol_to_dev(const float* zxy, void* yzx, int n_z, int n_x, int n_y, int fp64,
