@@ -270,14 +270,22 @@ __device__ __forceinline__ void table_step(const SweepArgs& A, const TabCtx<G, V
 
   // theta1 / theta2 (UpdateVoxels.cpp:343-369; BF: BFForwardModel.cpp:851-892)
   float t1 = 0.f, t2 = 0.f;
-  bool rejected = false;
+  // bit i * NB + b: selected before the update (kept where the registers are short), rejected
+  unsigned on0 = 0, rejected = 0;
+  auto was_on = [&](int i, int b) {
+    return kWide ? on0 >> (i * NB + b) & 1u : sv[BF ? i : 0][b];
+  };
   if constexpr (BF) {
 #pragma unroll
     for (int i = 0; i < VPL; ++i)
 #pragma unroll
-      for (int b = 0; b < NB; ++b) rejected |= f4_at(aq[i], b + 1) > 0.f && sv[i][b] == 0;
+      for (int b = 0; b < NB; ++b) {
+        const unsigned bit = 1u << (i * NB + b);
+        if (kWide && sv[i][b] != 0) on0 |= bit;
+        if (f4_at(aq[i], b + 1) > 0.f && sv[i][b] == 0) rejected |= bit;
+      }
   }
-  if (!BF || !__any_sync(kFull, rejected)) {
+  if (!BF || !__any_sync(kFull, rejected != 0)) {
 #pragma unroll
     for (int i = 0; i < VPL; ++i)
 #pragma unroll
@@ -292,7 +300,28 @@ __device__ __forceinline__ void table_step(const SweepArgs& A, const TabCtx<G, V
         }
       }
   } else if constexpr (BF) {
-    // entries that the selector rejects count with weight delta T / (|e| sqrt(w))
+    // entries that the selector rejects count with weight delta T / (|e| sqrt(w)): a root and a
+    // division, ~300 cycles of a chain that nothing overlaps.  The lanes take them together, each
+    // for its own next rejected entry, as often as one lane has rejected entries instead of once
+    // for each of its VPL * NB entries (20 calls at 75 views, T = 3: 14.5 -> 13.3 ms of sweep
+    // kernels; at 61 views 17.1 -> 15.9)
+    float qc[VPL * NB];
+#pragma unroll
+    for (int k = 0; k < VPL * NB; ++k) qc[k] = 0.f;
+    while (rejected) {
+      const unsigned bit = rejected & (0u - rejected);
+      rejected ^= bit;
+      float e = 0.f, w = 0.f;
+#pragma unroll
+      for (int k = 0; k < VPL * NB; ++k) {
+        e = bit == (1u << k) ? ev[k / NB][k % NB] : e;
+        w = bit == (1u << k) ? wv[k / NB][k % NB] : w;
+      }
+      const float q = c.bdt / (fabsf(e) * sqrtf(w));
+#pragma unroll
+      for (int k = 0; k < VPL * NB; ++k) qc[k] = bit == (1u << k) ? q : qc[k];
+    }
+    __syncwarp();
 #pragma unroll
     for (int i = 0; i < VPL; ++i)
 #pragma unroll
@@ -301,13 +330,12 @@ __device__ __forceinline__ void table_step(const SweepArgs& A, const TabCtx<G, V
         const float w = wv[i][b];
         const float pe = c.gx[i] * a * c.hh;
         if (a > 0.f) {
-          if (sv[i][b]) {
+          if (was_on(i, b)) {
             t2 += pe * pe * w;
             t1 += ev[i][b] * pe * w;
           } else {
-            const float qc = c.bdt / (fabsf(ev[i][b]) * sqrtf(w));
-            t2 += qc * (pe * pe * w);
-            t1 += qc * (ev[i][b] * pe * w);
+            t2 += qc[i * NB + b] * (pe * pe * w);
+            t1 += qc[i * NB + b] * (ev[i][b] * pe * w);
           }
         }
       }
@@ -348,7 +376,7 @@ __device__ __forceinline__ void table_step(const SweepArgs& A, const TabCtx<G, V
             // call's time at 1024 bins and 121 views); in shared memory the test costs more than
             // the store (19.0 against 17.1 ms of sweep kernels per equivalent iteration)
             const unsigned on = bragg_selected<float>(ne, wv[i][b], c.bt);
-            if (STAGE || on != sv[i][b]) c.bs[c.soff[i] + j + b] = static_cast<uint8_t>(on);
+            if (STAGE || on != was_on(i, b)) c.bs[c.soff[i] + j + b] = static_cast<uint8_t>(on);
           }
         }
       }
