@@ -669,12 +669,6 @@ __global__ void __launch_bounds__(1024)
   if (tid == 0) *n_vis = base;
 }
 
-__global__ void nh_mask_kernel(const double* __restrict__ filt, double thr,
-                               uint8_t* __restrict__ active, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) active[i] = filt[i] > thr ? 1 : 0;
-}
-
 // ROI sums: kind 0 = sum of the magnitude map over ROI lines, kind 1 = sum of the volume over
 // ROI lines and all y.  The ROI is the index box [x0,x1] x [z0,z1].
 template <typename Real>
@@ -897,12 +891,6 @@ int launch_bf_nh_list(const double* filt, const uint8_t* lineok, int n, int rank
                       unsigned long long* fx, int* vis, int* n_vis, void* stream) {
   nh_list_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(filt, lineok, n, rank, active,
                                                                     fx, vis, n_vis);
-  return ok_or(cudaGetLastError());
-}
-
-int launch_bf_nh_mask(const double* filt, double thr, uint8_t* active, int n, void* stream) {
-  nh_mask_kernel<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(filt, thr, active,
-                                                                                n);
   return ok_or(cudaGetLastError());
 }
 

@@ -318,7 +318,6 @@ int launch_bf_h_list(const uint8_t* slot, int j, uint8_t* active, unsigned long 
 // the lines above the order statistic `rank` of filt: mask, magnitudes cleared, ascending list
 int launch_bf_nh_list(const double* filt, const uint8_t* lineok, int n, int rank, uint8_t* active,
                       unsigned long long* fx, int* vis, int* n_vis, void* stream);
-int launch_bf_nh_mask(const double* filt, double thr, uint8_t* active, int n, void* stream);
 int launch_roi_sum(const DevGeom& g, int exact, int kind, const double* mag, const void* x,
                    int fp64, double* partial, double* out, void* stream);
 
