@@ -180,6 +180,55 @@ __device__ __forceinline__ float weight_times(float w, double a, wide::F2 af) {
   return r;
 }
 
+// The terms of the entries that the selector rejects, with FP64 roots and divisions (~40
+// operations, each 16 cycles of the SM per warp however few lanes take part).  A warp collects such
+// entries of detector rows [t0, t1) and evaluates 32 at a time (20 offset and 20 variance updates
+// at 75 x 333 x 97 entries with T = 3, with the division of the sums moved into the passes: 6.4 ->
+// 4.7 ms).
+template <int KIND>
+__device__ __forceinline__ void rejected_sums(const float* __restrict__ e, const float* w,
+                                              const uint8_t* __restrict__ sel, double a,
+                                              wide::F2 af, int store, double T, double dl, int v,
+                                              int t0, int t1, int n_theta, int n_rp, int n_sp,
+                                              int n_r, double (&acc)[2]) {
+  __shared__ float2 queue[8][64];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float2* q = queue[warp];
+  auto term = [&](float2 ew) {
+    if constexpr (KIND == kOffsetSums)
+      offset_term(ew.x, ew.y, false, T, dl, acc[0], acc[1]);
+    else if constexpr (KIND == kVarianceSums)
+      variance_term(ew.x, ew.y, a, false, acc[0], acc[1]);
+    else
+      acc[0] += cost_term(ew.x, ew.y, false, T, dl);
+  };
+  const int n = (t1 - t0) * n_r;
+  int held = 0;
+  for (int i0 = 32 * warp; i0 < n; i0 += 256) {
+    const int i = i0 + lane, dt = i / n_r, r = i - dt * n_r;
+    const size_t row = static_cast<size_t>(t0 + dt) * n_theta + v;
+    const bool off = i < n && sel[row * n_sp + r] != 1;
+    const unsigned m = __ballot_sync(0xffffffffu, off);
+    if (!m) continue;
+    if (off) {
+      float wv = w[row * n_rp + r];
+      if (KIND == kVarianceSums && !store) wv = weight_times(wv, a, af);
+      q[held + __popc(m & ((1u << lane) - 1u))] = make_float2(e[row * n_rp + r], wv);
+    }
+    held += __popc(m);
+    __syncwarp();
+    if (held >= 32) {
+      term(q[lane]);
+      held -= 32;
+      const float2 next = q[32 + lane];
+      __syncwarp();
+      if (lane < held) q[lane] = next;
+      __syncwarp();
+    }
+  }
+  if (lane < held) term(q[lane]);
+}
+
 template <int KIND>
 __global__ void __launch_bounds__(256)
     sums_f32_kernel(const float* __restrict__ e, float* __restrict__ w,
@@ -193,7 +242,7 @@ __global__ void __launch_bounds__(256)
   const wide::F2 af = wide::split(a);
   double acc[2] = {0.0, 0.0};
   wide::WideSum sum[2];
-  bool any = false;
+  bool any = false, rejected = false;
   wide::for_view_rows(
       v, t0, t1, n_theta, n_rp,
       [&](size_t row, int r) {
@@ -215,12 +264,8 @@ __global__ void __launch_bounds__(256)
             } else {
               sum[0].add(wide::mul(wide::two_prod(ev[j], ev[j]), wv[j]));
             }
-          } else if constexpr (KIND == kOffsetSums) {
-            offset_term(ev[j], wv[j], false, T, dl, acc[0], acc[1]);
-          } else if constexpr (KIND == kVarianceSums) {
-            variance_term(ev[j], wv[j], a, false, acc[0], acc[1]);
           } else {
-            acc[0] += cost_term(ev[j], wv[j], false, T, dl);
+            rejected = true;
           }
         }
         if constexpr (KIND == kVarianceSums) {
@@ -254,20 +299,26 @@ __global__ void __launch_bounds__(256)
         sum[1] = wide::WideSum();
         any = false;
       });
+  if (__syncthreads_or(rejected))
+    rejected_sums<KIND>(e, w, sel, a, af, store, T, dl, v, t0, t1, n_theta, n_rp, n_sp, n_r, acc);
   const double s = wide::block_sums<2>(acc);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (warp < 2 && lane == 0) partial[(static_cast<size_t>(v) * n_chunk + ch) * 2 + warp] = s;
 }
 
-// e -= step of the view, then the selector (offset_apply_kernel and selector_kernel)
+// e -= step of the view (its num / den of the offset sums, the host's division), then the selector
+// (offset_apply_kernel and selector_kernel)
 __global__ void __launch_bounds__(256)
     offset_step_f32_kernel(float* __restrict__ e, const float* __restrict__ w,
-                           uint8_t* __restrict__ sel, const double* __restrict__ step, double T,
+                           uint8_t* __restrict__ sel, const double* __restrict__ sums, double T,
                            int n_theta, int n_rp, int n_sp, int n_r, int n_t, int n_chunk) {
   const int v = blockIdx.x, ch = blockIdx.y;
   const int t0 = static_cast<int>(static_cast<long long>(ch) * n_t / n_chunk);
   const int t1 = static_cast<int>(static_cast<long long>(ch + 1) * n_t / n_chunk);
-  const double st = step[v], t2 = T * T;
+  __shared__ double s_step;
+  if (threadIdx.x == 0) s_step = sums[2 * v] / sums[2 * v + 1];
+  __syncthreads();
+  const double st = s_step, t2 = T * T;
   const wide::F2 sf = wide::neg(wide::split(st));
   const float t2f = static_cast<float>(t2);
   wide::for_view_rows(
@@ -304,14 +355,21 @@ __global__ void __launch_bounds__(256)
 // scale_weights_kernel and selector_kernel)
 __global__ void __launch_bounds__(256)
     new_weights_f32_kernel(const float* __restrict__ e, float* __restrict__ w,
-                           uint8_t* __restrict__ sel, const double* __restrict__ alpha, double upd,
-                           double T, int n_theta, int n_rp, int n_sp, int n_r, int n_t,
-                           int n_chunk) {
+                           uint8_t* __restrict__ sel, const double* __restrict__ alpha,
+                           const double* __restrict__ sums, double dT, double count, double T,
+                           int n_theta, int n_rp, int n_sp, int n_r, int n_t, int n_chunk) {
   const int v = blockIdx.x, ch = blockIdx.y;
   const int t0 = static_cast<int>(static_cast<long long>(ch) * n_t / n_chunk);
   const int t1 = static_cast<int>(static_cast<long long>(ch + 1) * n_t / n_chunk);
   const double a = alpha[v], t2 = T * T;
-  const wide::F2 af = wide::split(a), inv = wide::split(1.0 / upd);
+  __shared__ double s_upd[2];  // the new variance, once per block (FP64 divisions), its inverse
+  if (threadIdx.x == 0) {
+    s_upd[0] = (sums[0] + dT * sums[1]) / count;
+    s_upd[1] = 1.0 / s_upd[0];
+  }
+  __syncthreads();
+  const double upd = s_upd[0];
+  const wide::F2 af = wide::split(a), inv = wide::split(s_upd[1]);
   const float t2f = static_cast<float>(t2);
   wide::for_view_rows(
       v, t0, t1, n_theta, n_rp,
@@ -804,22 +862,22 @@ int launch_bf_variance_sums(const BfSino& b, int exact, const double* alpha, boo
 }
 
 // FP32 engine: the offset step and the selector that follows it, in one pass
-int launch_bf_offset_step(const BfSino& b, const double* step, double T, void* stream) {
+int launch_bf_offset_step(const BfSino& b, const double* sums, double T, void* stream) {
   const int chunks = view_chunks(b);
   offset_step_f32_kernel<<<dim3(b.n_theta, chunks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      RP<float>(b.e), RP<float>(b.w), b.sel, step, T, b.n_theta, b.n_rp, b.n_sp, b.n_r, b.n_t,
+      RP<float>(b.e), RP<float>(b.w), b.sel, sums, T, b.n_theta, b.n_rp, b.n_sp, b.n_r, b.n_t,
       chunks);
   return ok_or(cudaGetLastError());
 }
 
 // FP32 engine: the weights of the new common variance (after variance sums that did not scale
 // them) and the selector that follows, in one pass
-int launch_bf_new_weights(const BfSino& b, const double* alpha, double upd, double T,
-                          void* stream) {
+int launch_bf_new_weights(const BfSino& b, const double* alpha, const double* sums, double dT,
+                          double count, double T, void* stream) {
   const int chunks = view_chunks(b);
   new_weights_f32_kernel<<<dim3(b.n_theta, chunks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      RP<float>(b.e), RP<float>(b.w), b.sel, alpha, upd, T, b.n_theta, b.n_rp, b.n_sp, b.n_r, b.n_t,
-      chunks);
+      RP<float>(b.e), RP<float>(b.w), b.sel, alpha, sums, dT, count, T, b.n_theta, b.n_rp, b.n_sp,
+      b.n_r, b.n_t, chunks);
   return ok_or(cudaGetLastError());
 }
 

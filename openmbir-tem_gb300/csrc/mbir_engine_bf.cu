@@ -727,6 +727,9 @@ int Engine::bf_joint_estimation() {
   int rc = launch_bf_offset_sums(b, exact_ ? 1 : 0, bragg_t_, p_.bragg_delta, d_partial_,
                                  n_chunk_, d_vsum_, s);
   if (rc) return cuda_check(rc, "offset sums");
+  // the FP32 engine's step needs no host: its pass divides the sums itself
+  if (!fp64_ && (rc = launch_bf_offset_step(b, d_vsum_, bragg_t_, s)))
+    return cuda_check(rc, "offset step");
   std::vector<double> vs(static_cast<size_t>(nt) * 2), step(nt);
   cudaMemcpyAsync(vs.data(), d_vsum_, sizeof(double) * vs.size(), cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "offset sums");
@@ -734,14 +737,12 @@ int Engine::bf_joint_estimation() {
     step[v] = vs[v * 2 + 0] / vs[v * 2 + 1];
     mu_[v] += step[v];
   }
-  cudaMemcpyAsync(d_mu2_, step.data(), sizeof(double) * nt, cudaMemcpyHostToDevice, s);
   if (fp64_) {
+    cudaMemcpyAsync(d_mu2_, step.data(), sizeof(double) * nt, cudaMemcpyHostToDevice, s);
     if ((rc = launch_bf_offset_apply(b, d_mu2_, s))) return cuda_check(rc, "offset apply");
     if ((rc = launch_bf_selector(b, bragg_t_, s))) return cuda_check(rc, "selector");
-  } else {
-    if ((rc = launch_bf_offset_step(b, d_mu2_, bragg_t_, s))) return cuda_check(rc, "offset step");
+    if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "offset step");
   }
-  if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "offset step");
   return upload_views();
 }
 
@@ -754,18 +755,19 @@ int Engine::bf_update_weights() {
   cudaMemcpyAsync(d_alpha_, alpha_.data(), sizeof(double) * g.n_theta, cudaMemcpyHostToDevice, s);
   int rc = launch_bf_variance_sums(b, exact_ ? 1 : 0, d_alpha_, false, d_bfpart_, d_bfout_, s);
   if (rc) return cuda_check(rc, "variance sums");
+  const double dT = p_.bragg_delta * bragg_t_;
+  const int count = g.n_theta * g.n_r * g.n_t;
+  // (d_alpha_ still holds the variances before this update)
+  if (!fp64_ && (rc = launch_bf_new_weights(b, d_alpha_, d_bfout_, dT, count, bragg_t_, s)))
+    return cuda_check(rc, "new weights");
   double sums[2];
   cudaMemcpyAsync(sums, d_bfout_, sizeof(sums), cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "variance sums");
-  const double upd = (sums[0] + (p_.bragg_delta * bragg_t_) * sums[1]) /
-                     (g.n_theta * g.n_r * g.n_t);
+  const double upd = (sums[0] + dT * sums[1]) / count;
   for (int v = 0; v < g.n_theta; v++) alpha_[v] = upd;
   if (fp64_) {
     if ((rc = launch_bf_scale_weights(b, upd, s))) return cuda_check(rc, "weight scale");
     if ((rc = launch_bf_selector(b, bragg_t_, s))) return cuda_check(rc, "selector");
-  } else {  // (d_alpha_ still holds the variances before this update)
-    if ((rc = launch_bf_new_weights(b, d_alpha_, upd, bragg_t_, s)))
-      return cuda_check(rc, "new weights");
   }
   cudaMemcpyAsync(d_alpha_, alpha_.data(), sizeof(double) * g.n_theta, cudaMemcpyHostToDevice, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_check(MBIR_EDEVICE, "variance");

@@ -304,8 +304,11 @@ int launch_bf_selector(const BfSino& b, double T, void* stream);
 // scale: the weights become w alpha (the exact mode and the FP64 engine always do that)
 int launch_bf_variance_sums(const BfSino& b, int exact, const double* alpha, bool scale,
                             double* partial, double* out, void* stream);
-int launch_bf_offset_step(const BfSino& b, const double* step, double T, void* stream);
-int launch_bf_new_weights(const BfSino& b, const double* alpha, double upd, double T, void* stream);
+// the offset step of each view from its sums [n_theta][2]; the weights with the new variance
+// (sums[0] + dT sums[1]) / count
+int launch_bf_offset_step(const BfSino& b, const double* sums, double T, void* stream);
+int launch_bf_new_weights(const BfSino& b, const double* alpha, const double* sums, double dT,
+                          double count, double T, void* stream);
 int launch_bf_scale_weights(const BfSino& b, double alpha, void* stream);
 int launch_bf_cost_sums(const BfSino& b, int exact, double T, double dl, double* partial,
                         double* out, void* stream);
