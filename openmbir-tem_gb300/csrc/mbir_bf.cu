@@ -176,7 +176,7 @@ __device__ __forceinline__ float weight_times(float w, double a, wide::F2 af) {
   const wide::F2 p = wide::mul(af, w);
   float r;
   if (!wide::rounds_to(p, 1.2e-13f * fabsf(p.hi), r))
-    r = static_cast<float>(static_cast<double>(w) * a);
+    r = wide::times_fp64(w, a);
   return r;
 }
 
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(256)
           const wide::F2 d = wide::add(wide::two_sum(ev[j], sf.hi), wide::F2{sf.lo, 0.f});
           float o;
           if (!wide::rounds_to(d, 1.2e-13f * (fabsf(ev[j]) + fabsf(sf.hi)), o))
-            o = static_cast<float>(static_cast<double>(ev[j]) - st);
+            o = wide::minus_fp64(ev[j], st);
           ev[j] = o;
           on[j] = wide::below(o, wv[j], t2, t2f) ? 1 : 0;
         }
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(256)
           const float w1 = weight_times(wv[j], a, af);
           const wide::F2 q = wide::mul(inv, w1);
           if (!wide::rounds_to(q, 1.2e-13f * fabsf(q.hi), wv[j]))
-            wv[j] = static_cast<float>(static_cast<double>(w1) / upd);
+            wv[j] = wide::over_fp64(w1, upd);
           on[j] = wide::below(ev[j], wv[j], t2, t2f) ? 1 : 0;
         }
         *reinterpret_cast<float4*>(w + base + r) = make_float4(wv[0], wv[1], wv[2], wv[3]);
