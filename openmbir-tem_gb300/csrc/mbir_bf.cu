@@ -623,8 +623,10 @@ __global__ void h_list_kernel(const uint8_t* __restrict__ slot, int j, uint8_t* 
 // the top, until the bucket holds at most kTail values, which are then ranked directly; then the
 // active mask, the magnitudes' restart and the ascending list of the active lines with an
 // A-column.  On the host (read-back of the map, nth_element, list, upload) this took ~0.25 ms of
-// a call's 2.1 on 512 x 128 lines; here ~0.03.
-constexpr int kTail = 1024;
+// a call's 2.1 on 512 x 128 lines; with one load in flight per thread 0.217 ms, with kAtOnce and a
+// tail of 256 instead of 1024 values 0.104 (under a profiler, caches cold; a call took 0.09 less).
+constexpr int kTail = 256;
+constexpr int kAtOnce = 8;  // loads of a thread in flight: one SM reads the values, latency counts
 __global__ void __launch_bounds__(1024)
     nh_list_kernel(const double* __restrict__ filt, const uint8_t* __restrict__ lineok, int n,
                    int rank, uint8_t* __restrict__ active, unsigned long long* __restrict__ fx,
@@ -633,7 +635,7 @@ __global__ void __launch_bounds__(1024)
   __shared__ unsigned long long tail[kTail];
   __shared__ unsigned long long s_prefix;
   __shared__ int s_rank, s_count, s_n;
-  __shared__ int warp_n[32];
+  __shared__ int before[kAtOnce][32], row_n[kAtOnce];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned long long* bits = reinterpret_cast<const unsigned long long*>(filt);
   unsigned long long prefix = 0ull;  // the bits above `shift + 8` of the order statistic
@@ -642,14 +644,22 @@ __global__ void __launch_bounds__(1024)
     shift -= 8;
     if (tid < 256) hist[tid] = 0;
     __syncthreads();
-    for (int i0 = 0; i0 < n; i0 += 1024) {
-      const int i = i0 + tid;
-      const unsigned long long v = i < n ? bits[i] : 0ull;
-      const bool in = i < n && (shift == 56 || (v >> (shift + 8)) == prefix);
-      const int d = in ? static_cast<int>((v >> shift) & 255u) : -1;
-      // the values of a warp share their upper digits: one addition per distinct digit
-      const unsigned same = __match_any_sync(0xffffffffu, d);
-      if (in && lane == __ffs(same) - 1) atomicAdd(&hist[d], __popc(same));
+    for (int i0 = 0; i0 < n; i0 += kAtOnce * 1024) {
+      unsigned long long v[kAtOnce];
+#pragma unroll
+      for (int k = 0; k < kAtOnce; ++k) {
+        const int i = i0 + k * 1024 + tid;
+        v[k] = i < n ? bits[i] : 0ull;
+      }
+#pragma unroll
+      for (int k = 0; k < kAtOnce; ++k) {
+        const bool in = i0 + k * 1024 + tid < n && (shift == 56 || (v[k] >> (shift + 8)) == prefix);
+        if (!__any_sync(0xffffffffu, in)) continue;
+        const int d = in ? static_cast<int>((v[k] >> shift) & 255u) : -1;
+        // the values of a warp share their upper digits: one addition per distinct digit
+        const unsigned same = __match_any_sync(0xffffffffu, d);
+        if (in && lane == __ffs(same) - 1) atomicAdd(&hist[d], __popc(same));
+      }
     }
     __syncthreads();
     if (warp == 0) {  // the bucket of rank r: eight digits per lane, summed across the warp
@@ -685,9 +695,17 @@ __global__ void __launch_bounds__(1024)
   if (shift > 0) {  // rank the bucket's values
     if (tid == 0) s_n = 0;
     __syncthreads();
-    for (int i = tid; i < n; i += 1024) {
-      const unsigned long long v = bits[i];
-      if (shift == 64 || (v >> shift) == prefix) tail[atomicAdd(&s_n, 1)] = v;
+    for (int i0 = 0; i0 < n; i0 += kAtOnce * 1024) {
+      unsigned long long v[kAtOnce];
+#pragma unroll
+      for (int k = 0; k < kAtOnce; ++k) {
+        const int i = i0 + k * 1024 + tid;
+        v[k] = i < n ? bits[i] : 0ull;
+      }
+#pragma unroll
+      for (int k = 0; k < kAtOnce; ++k)
+        if (i0 + k * 1024 + tid < n && (shift == 64 || (v[k] >> shift) == prefix))
+          tail[atomicAdd(&s_n, 1)] = v[k];
     }
     __syncthreads();
     if (tid < count) {
@@ -704,24 +722,44 @@ __global__ void __launch_bounds__(1024)
   }
   const double thr = __longlong_as_double(static_cast<long long>(prefix));
   int base = 0;
-  for (int i0 = 0; i0 < n; i0 += 1024) {
-    const int i = i0 + tid;
-    const bool on = i < n && filt[i] > thr;
-    if (i < n) {
-      active[i] = on ? 1 : 0;
+  for (int i0 = 0; i0 < n; i0 += kAtOnce * 1024) {
+    double f[kAtOnce];
+    uint8_t ok[kAtOnce];
+#pragma unroll
+    for (int k = 0; k < kAtOnce; ++k) {
+      const int i = i0 + k * 1024 + tid;
+      f[k] = i < n ? filt[i] : 0.0;
+      ok[k] = i < n ? lineok[i] : 0;
+    }
+    unsigned m[kAtOnce];
+#pragma unroll
+    for (int k = 0; k < kAtOnce; ++k) {
+      const int i = i0 + k * 1024 + tid;
+      const bool on = i < n && f[k] > thr;
+      if (i < n) active[i] = on ? 1 : 0;
       if (on) fx[i] = 0ull;
+      m[k] = __ballot_sync(0xffffffffu, on && ok[k] != 0);
+      if (lane == 0) before[k][warp] = __popc(m[k]);
     }
-    const bool in = on && lineok[i] != 0;
-    const unsigned b = __ballot_sync(0xffffffffu, in);
-    if (lane == 0) warp_n[warp] = __popc(b);
     __syncthreads();
-    int at = base + __popc(b & ((1u << lane) - 1u)), all = 0;
-    for (int w = 0; w < 32; ++w) {
-      at += w < warp ? warp_n[w] : 0;
-      all += warp_n[w];
+    if (warp < kAtOnce) {  // the lines of the warps before, row by row
+      const int c = before[warp][lane];
+      int sum = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += u;
+      }
+      before[warp][lane] = sum - c;
+      if (lane == 31) row_n[warp] = sum;
     }
-    if (in) vis[at] = i;
-    base += all;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kAtOnce; ++k) {
+      if (m[k] >> lane & 1u)
+        vis[base + before[k][warp] + __popc(m[k] & ((1u << lane) - 1u))] = i0 + k * 1024 + tid;
+      base += row_n[k];
+    }
     __syncthreads();
   }
   if (tid == 0) *n_vis = base;

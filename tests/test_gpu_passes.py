@@ -10,8 +10,7 @@ from test_gpu_table import rel, series
 pytestmark = pytest.mark.gpu
 
 
-# lines below, at and above the 1024 that the last step of the selection ranks at once; most
-# magnitudes of the first calls are zeros, so that the order statistic lies among ties
+# fewer lines than the last step of the selection ranks at once, and more; most magnitudes of the first calls are zeros, so that the order statistic lies among ties
 @pytest.mark.parametrize("n_r,n_t,thickness", [(12, 2, 6.0), (64, 2, 16.0), (65, 3, 16.0),
                                                (96, 2, 24.0)])
 def test_nonhomogeneous_lists(lib_built, n_r, n_t, thickness):
