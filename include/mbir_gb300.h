@@ -361,7 +361,7 @@ int32_t mbir_run_multires(const mbir_params* p, const float* counts, const float
                           double delta_t, float* out, int64_t n, int32_t* dims_out);
 
 /* Batched execution (config "many uneven reconstructions"): prepared FP32 parallel-order
- * engines on one device advance together, one persistent cooperative launch per ICD sweep
+ * engines on one device advance together, persistent launches side by side per ICD sweep
  * covering every voxel slice of every engine; gain/offset, variance and cost stay per engine.
  * The reference has no counterpart: it runs one reconstruction per process
  * (HAADF_MultiResolutionReconstruction.cpp:175-485). */
