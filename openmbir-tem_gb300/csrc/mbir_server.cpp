@@ -146,16 +146,17 @@ int Server::admit_locked(std::vector<Request*>& admitted) {
   while (!queue_.empty() && static_cast<int>(active_.size() + prepared_.size() + preparing_ +
                                              admitted.size()) < max_active_) {
     Request* r = queue_.front();
-    if (used_ + static_cast<int64_t>(r->bytes) > budget_) break;  // arrival order: no overtaking
+    if (used_ + tables_ + static_cast<int64_t>(r->bytes) > budget_) break;  // arrival order: no overtaking
     queue_.pop_front();
     // tables take at most half of the budget, and none that a queued request's own arrays need
     const size_t table = table_bytes(*r);
     int64_t queued = 0;
     for (const Request* q : queue_) queued += static_cast<int64_t>(q->bytes);
-    const int64_t with = used_ + static_cast<int64_t>(r->bytes + table);
+    const int64_t with = used_ + tables_ + static_cast<int64_t>(r->bytes + table);
     const bool room = with + queued <= budget_ && with <= budget_ / 2;
     r->engine->allow_table(room);
-    if (room) r->bytes += table;
+    r->table = room ? static_cast<int64_t>(table) : 0;
+    tables_ += r->table;
     used_ += static_cast<int64_t>(r->bytes);
     admitted.push_back(r);
     stats_.admitted++;
@@ -175,6 +176,7 @@ void Server::retire(Request* r, int code, const std::string& msg) {
   r->state = code == 0 ? 2 : code;
   r->error = msg;
   used_ -= static_cast<int64_t>(r->bytes);
+  tables_ -= r->table;
   if (code == 0) {
     stats_.completed++;
     latencies_ms_.push_back((r->t_done - r->t_submit) * 1e3);

@@ -27,7 +27,8 @@ struct Request {
   double t_submit = 0, t_admit = 0, t_done = 0;  // seconds (steady clock)
   int outer_done = 0;
   double cost = 0, prev_cost = 0;
-  size_t bytes = 0;
+  size_t bytes = 0;   // its own arrays
+  int64_t table = 0;  // its A-column table, 0 without one
   std::unique_ptr<Engine> engine;
   std::vector<float> result;  // [z][x][y]
   int dims[3] = {0, 0, 0};
@@ -73,7 +74,8 @@ class Server {
   int device_;
   int64_t budget_;
   int max_active_;
-  int64_t used_ = 0;
+  int64_t used_ = 0;    // of the admitted requests' own arrays (peak_bytes is its maximum)
+  int64_t tables_ = 0;  // of their tables; used_ + tables_ stays within the budget
   int64_t last_admitted_id_ = 0;
   int64_t next_id_ = 1;
   mutable std::mutex mu_;
