@@ -178,12 +178,21 @@ int Batch::sweep(const std::vector<std::pair<int, int>>& iters, double* stats) {
   for (int i = 0; i < n; i++) {
     if (nb < 0) nb = eng_[i]->nb();
     if (eng_[i]->nb() != nb) return fail(MBIR_ENOTSUP, "batch: engines at different voxel sizes");
-    size_t need = eng_[i]->walk_smem_bytes(args[i], stage_cap);
-    if (args[i].smem_rows && need > stage_cap) {
-      args[i].smem_rows = 0;
-      args[i].n_rs = 0;
-      need = eng_[i]->walk_smem_bytes(args[i], stage_cap);
+    SweepArgs& a = args[i];
+    const float4* const acol = a.acol;
+    auto plan = [&](size_t limit) {
+      a.acol = acol;
+      return a.sched_lines != nullptr && table_driven(a, nb) ? eng_[i]->sched_smem_bytes(a)
+                                                             : eng_[i]->plan_walk(a, limit);
+    };
+    size_t need = plan(stage_cap);
+    if (a.smem_rows && need > stage_cap) {
+      a.smem_rows = 0;
+      a.n_rs = 0;
+      need = plan(stage_cap);
     }
+    // in place the slice may take the SM's whole shared memory
+    if (!a.smem_rows && a.acol != acol) need = plan(static_cast<size_t>(max_optin) - 2048);
     const int sh = (args[i].shape >= 1 && args[i].shape <= 4) ? args[i].shape : 4;
     groups[i] = batch_group(sh, args[i].bf != 0, table_driven(args[i], nb), args[i].smem_rows != 0);
     smem[groups[i]] = std::max(smem[groups[i]], need);

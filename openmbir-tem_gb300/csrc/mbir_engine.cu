@@ -1057,26 +1057,28 @@ void Engine::table_args(SweepArgs& a) const {
   a.pf.alpha = static_cast<float>(flt_.mrf_alpha);
 }
 
-// Dynamic shared memory of a launch that walks the rows; table-driven launches take two row
-// caches when they fit in `limit`
-size_t Engine::walk_smem_bytes(const SweepArgs& a, size_t limit) const {
+// Dynamic shared memory of a launch that walks the rows within `limit` (0: one CTA's).  The
+// table-driven layout takes ~62 bytes per voxel of a row, the general one 58 and 284 per view, so
+// with few views and rows of thousands of voxels (staged slices at 9 views: 2365 to 2424; in HBM at
+// 21 views: 3753 to 3866) only the general one fits: such a launch leaves the table aside.
+size_t Engine::plan_walk(SweepArgs& a, size_t limit) const {
   const bool staged = a.smem_rows != 0;
-  if (!table_driven(a, nb_))
-    return staged == stage_ ? smem_bytes_
-                            : sweep_smem_bytes(g_.n_theta, g_.n_x, 0, t_rows_, bins_, fp64_, 0);
-  const int n_sp = a.bf ? n_sp_ : 0;
-  const bool project = a.mode == kModeProject;
   if (limit == 0) limit = static_cast<size_t>(smem_optin_limit()) - 1024;
-  const size_t two =
-      table_smem_bytes(g_.n_theta, g_.n_x, a.n_rs, staged, n_sp, project, 2);
-  return two <= limit ? two
-                      : table_smem_bytes(g_.n_theta, g_.n_x, a.n_rs, staged, n_sp, project, 1);
+  if (table_driven(a, nb_)) {
+    const size_t bytes = table_walk_bytes(g_.n_theta, g_.n_x, a.n_rs, staged, a.bf ? n_sp_ : 0,
+                                          a.mode == kModeProject, limit);
+    if (bytes) return bytes;
+    a.acol = nullptr;
+  }
+  return staged == stage_ ? smem_bytes_
+                          : sweep_smem_bytes(g_.n_theta, g_.n_x, 0, t_rows_, bins_, fp64_, 0);
 }
 
-// Dynamic shared memory of a scheduled bright-field call, without the schedule itself
+// Dynamic shared memory of a scheduled bright-field call, without the schedule itself (its layout
+// has no rows, so that it fits wherever the general one does)
 size_t Engine::sched_smem_bytes(const SweepArgs& a) const {
   return table_driven(a, nb_)
-             ? table_smem_bytes(g_.n_theta, 0, a.n_rs, a.smem_rows != 0, n_sp_, false, 1)
+             ? table_smem_bytes(g_.n_theta, 0, a.n_rs, a.smem_rows != 0, n_sp_, false, 2)
              : smem_sched_bytes_;
 }
 
@@ -1117,11 +1119,12 @@ int Engine::forward_project() {
   a.stats = nullptr;
   a.err = d_err_;
   table_args(a);
+  const size_t smem = plan_walk(a);
   for (int colour = 0; colour < 2; colour++) {
     a.colour = colour;
     a.n_slices = (g.n_y - colour + 1) / 2;
     if (a.n_slices <= 0) continue;
-    int rc = launch_sweep(a, nb_, walk_smem_bytes(a), s);
+    int rc = launch_sweep(a, nb_, smem, s);
     if (rc) return cuda_check(rc, "forward projection launch");
   }
   int rc;
@@ -1236,6 +1239,7 @@ int Engine::sweep(int outer, int inner, double* stats4) {
       a.bf = 1;
       a.bfa = bfa_sweep_args();
     }
+    const size_t smem = plan_walk(a);
     const int n0 = (g.n_y + 1) / 2;
     cudaEventRecord(static_cast<cudaEvent_t>(ev2_), s);
     for (int colour = 0; colour < 2; colour++) {
@@ -1243,8 +1247,7 @@ int Engine::sweep(int outer, int inner, double* stats4) {
       a.n_slices = (g.n_y - colour + 1) / 2;
       a.stats = d_stats_ + (colour ? static_cast<size_t>(n0) * kStatSlots : 0);
       if (a.n_slices <= 0) continue;
-      if ((rc = launch_sweep(a, nb_, walk_smem_bytes(a), s)))
-        return cuda_check(rc, "ICD sweep launch");
+      if ((rc = launch_sweep(a, nb_, smem, s))) return cuda_check(rc, "ICD sweep launch");
     }
     cudaEventRecord(static_cast<cudaEvent_t>(ev3_), s);
     kernel_timed_ = true;
@@ -2033,6 +2036,7 @@ int Engine::autotune_shape() {
     a.bfa.bragg_t = bragg_t_;
     a.bfa.bragg_dt = p_.bragg_delta * bragg_t_;
   }
+  const size_t smem = plan_walk(a);
   const int n0 = (g.n_y + 1) / 2;
   int best = shape_;
   float best_ms = 0;
@@ -2048,7 +2052,7 @@ int Engine::autotune_shape() {
       a.colour = colour;
       a.n_slices = (g.n_y - colour + 1) / 2;
       a.stats = d_stats_ + (colour ? static_cast<size_t>(n0) * kStatSlots : 0);
-      if (a.n_slices > 0) rc = launch_sweep(a, nb_, walk_smem_bytes(a), s);
+      if (a.n_slices > 0) rc = launch_sweep(a, nb_, smem, s);
     }
     cudaEventRecord(static_cast<cudaEvent_t>(ev1_), s);
     // restore the state for the next candidate (and for the reconstruction itself)

@@ -168,11 +168,13 @@ class Engine {
   const Geometry& geometry() const { return g_; }
 
   // Hooks for the batched sweep (mbir_batch.cu).  batch_args fills the sweep arguments of this
-  // engine's next parallel-order sweep (uploading its row order); walk_smem_bytes is the shared
-  // memory of its slices as the arguments stage them (two row caches only within `limit`);
+  // engine's next parallel-order sweep (uploading its row order); plan_walk is the shared memory of
+  // a launch that walks the rows, staged as the arguments say, and takes the table out of them
+  // where its layout does not fit `limit`; sched_smem_bytes that of a scheduled call;
   // batch_finish records a sweep that ran inside a batch.
   int batch_args(int outer, int inner, SweepArgs* out);
-  size_t walk_smem_bytes(const SweepArgs& a, size_t limit = 0) const;
+  size_t plan_walk(SweepArgs& a, size_t limit = 0) const;
+  size_t sched_smem_bytes(const SweepArgs& a) const;
   int batch_finish(int outer, int inner, const double* st4, double ms);
   double* slice_stats() const { return d_stats_; }
   double* sweep_stats() const { return d_stat4_; }
@@ -202,7 +204,6 @@ class Engine {
   int build_acol();
   size_t acol_bytes() const;
   void table_args(SweepArgs& a) const;
-  size_t sched_smem_bytes(const SweepArgs& a) const;
   int host_footprint_bins();                      // acol_lo_, acol_mask_ (once, on demand)
   int bf_schedule(const std::vector<int32_t>& rows, SweepArgs& a);  // the call's levels
   void bf_schedule_readback();                    // queue the device schedule's copy to host

@@ -704,7 +704,7 @@ int Engine::bf_parallel_args(int iter_nonzero, const DevBF& bfa, SweepArgs* out,
   a.shape = shape_;
   table_args(a);
   if ((rc = bf_schedule(rows, a))) return rc;
-  size_t smem = a.sched_lines != nullptr ? sched_smem_bytes(a) : walk_smem_bytes(a);
+  size_t smem = a.sched_lines != nullptr ? sched_smem_bytes(a) : plan_walk(a);
   if (a.sched_lines != nullptr) {
     // room for the schedule itself (offsets and lines) after the layout, when it fits: the
     // class steps then read it from shared memory

@@ -337,6 +337,9 @@ int launch_table_haadf(const SweepArgs& a, size_t smem_bytes, void* stream);
 int launch_table_bf(const SweepArgs& a, size_t smem_bytes, void* stream);
 size_t table_smem_bytes(int n_theta, int n_x, int n_rs, bool stage, int n_sp, bool project,
                         int nbuf);
+// of a row walk within `limit` bytes: with two row caches, else with one, 0 when neither fits
+size_t table_walk_bytes(int n_theta, int n_x, int n_rs, bool stage, int n_sp, bool project,
+                        size_t limit);
 // sched: the layout of a scheduled bright-field call (smaller: no response table or row lists)
 size_t sweep_smem_bytes(int n_theta, int n_x, int n_rs, int t_rows, int bins, int fp64,
                         int n_sp, bool sched = false);

@@ -89,7 +89,7 @@ int Engine::sweep_colour(int colour, int outer, int inner, double* st4) {
   a.shape = shape_;
   a.err = d_err_;
   table_args(a);
-  size_t smem = walk_smem_bytes(a);
+  size_t smem = plan_walk(a);
   if (bf_) {
     a = slab_args_;
     smem = slab_smem_;

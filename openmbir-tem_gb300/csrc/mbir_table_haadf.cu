@@ -12,4 +12,13 @@ size_t table_smem_bytes(int n_theta, int n_x, int n_rs, bool stage, int n_sp, bo
   return sweep::table_layout(n_theta, n_x, n_rs, stage, n_sp, project, nbuf).total;
 }
 
+size_t table_walk_bytes(int n_theta, int n_x, int n_rs, bool stage, int n_sp, bool project,
+                        size_t limit) {
+  for (int nbuf = 2; nbuf > 0; --nbuf) {
+    const size_t b = table_smem_bytes(n_theta, n_x, n_rs, stage, n_sp, project, nbuf);
+    if (b <= limit) return b;
+  }
+  return 0;
+}
+
 }  // namespace mbir
