@@ -5,9 +5,10 @@
 // pipe takes 2 lanes per clock and SM, so 5 to 30 FP64 operations per element (conversions among
 // them) bound those passes at 5 to 30 times their memory time.  Here
 //   * sums use the error-free transformations of Knuth (two_sum) and Dekker/FMA (two_prod):
-//     WideSum holds a sum as three FP32 numbers whose rounding error is near 2^-70 of the sum, and
-//     is added to an FP64 accumulator once per thread and chunk, so that fewer FP64 roundings
-//     take part than when every term was added in FP64;
+//     a product of two or three FP32 numbers enters as the pairs whose sum it is exactly, WideSum
+//     holds the sum as three FP32 numbers whose rounding error is near 2^-70 of it, and is added
+//     to an FP64 accumulator once per thread and chunk, so that fewer FP64 roundings take part than
+//     when every term was multiplied and added in FP64;
 //   * elementwise results are computed to ~2^-44 and rounded to FP32 when no rounding boundary is
 //     near (Ziv's test); otherwise, about once in 10^5 elements, the FP64 expression is evaluated.
 //     Results are the same bits as the FP64 expression's.
