@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(256)
   const int t0 = static_cast<int>(static_cast<long long>(ch) * n_t / n_chunk);
   const int t1 = static_cast<int>(static_cast<long long>(ch + 1) * n_t / n_chunk);
   const double a = KIND == kVarianceSums ? alpha[v] : 1.0;
-  const wide::F2 af = wide::split(a);
+  const wide::F2 af = wide::split_factor(a);
   double acc[2] = {0.0, 0.0};
   wide::WideSum sum[2];
   bool any = false, rejected = false;
@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(256)
   }
   __syncthreads();
   const double upd = s_upd[0];
-  const wide::F2 af = wide::split(a), inv = wide::split(s_upd[1]);
+  const wide::F2 af = wide::split_factor(a), inv = wide::split_factor(s_upd[1]);
   const float t2f = static_cast<float>(t2);
   wide::for_view_rows(
       v, t0, t1, n_theta, n_rp,

@@ -56,6 +56,11 @@ __device__ __forceinline__ F2 split(double v) {
   const float h = static_cast<float>(v);
   return {h, static_cast<float>(v - static_cast<double>(h))};
 }
+// v as a factor of a product that is rounded to FP32 (rounds_to): below 2^-90 the low part would be
+// subnormal and short of bits, so a product takes the FP64 expression there (no F2 rounds with NaN)
+__device__ __forceinline__ F2 split_factor(double v) {
+  return fabs(v) >= 8.1e-28 ? split(v) : F2{__int_as_float(0x7fc00000), 0.f};
+}
 
 struct WideSum {
   float s0 = 0.f, s1 = 0.f, s2 = 0.f;
@@ -114,9 +119,10 @@ static __device__ __noinline__ float times_fp64(float w, double by) {
 
 // e^2 w < t2 as the FP64 expression decides it; t2f = (float)t2
 __device__ __forceinline__ bool below(float e, float w, double t2, float t2f) {
-  const float p = __fmul_rn(__fmul_rn(e, e), w);
-  // FP32 product within 2^-22 of the true one unless it under- or overflows
-  if (p >= 1e-30f && p <= 1e36f && (t2f > 1e38f || fabsf(__fsub_rn(p, t2f)) > 1e-6f * t2f))
+  const float q = __fmul_rn(e, e), p = __fmul_rn(q, w);
+  // FP32 product within 2^-22 of the true one unless it or e^2 under- or overflows
+  if (q >= 1e-30f && p >= 1e-30f && p <= 1e36f &&
+      (t2f > 1e38f || fabsf(__fsub_rn(p, t2f)) > 1e-6f * t2f))
     return p < t2f;
   return below_fp64(e, w, t2);
 }
