@@ -132,23 +132,8 @@ __global__ void error_from_projection_kernel(const Real* __restrict__ y,
 // The gain/offset solve subtracts these sums from one another and a sweep's zero skipping turns a
 // last-bit difference of its inputs into another path, so every rounding of the sums is kept.
 // The FP64 pipe bounds the kernel (2 lanes per clock and SM): kind 0 took ~23 FP64 operations per
-// entry, ~10 of them the division by the view's gain.  div_by gives the same quotient in five;
-// the FP32 engine leaves out sum y^2 w (Y2 false), which its solve does not use.
-
-// x / g, correctly rounded, from inv = rn(1 / g): one refinement makes the quotient faithful, a
-// second one correctly rounded (Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", 1990), for magnitudes far from the ends of the exponent range
-__device__ __forceinline__ bool mid_range(double x) {
-  const unsigned e = (static_cast<unsigned>(__double2hiint(x)) >> 20) & 0x7ffu;
-  return e - 400u < 1247u;  // 2^-623 <= |x| < 2^624
-}
-__device__ __forceinline__ double div_by(double x, double g, double inv, bool mid) {
-  if (!mid || !mid_range(x)) return x / g;
-  double q = x * inv;
-  q = fma(fma(-q, g, x), inv, q);
-  return fma(fma(-q, g, x), inv, q);
-}
-
+// entry, ~10 of them the division by the view's gain.  wide::div_by gives the same quotient in
+// five; the FP32 engine leaves out sum y^2 w (Y2 false), which its solve does not use.
 template <typename Real, int K, bool Y2>
 __global__ void view_sums_kernel(const Real* __restrict__ y, const Real* __restrict__ e,
                                  const double* __restrict__ mu, const double* __restrict__ gain,
@@ -164,8 +149,7 @@ __global__ void view_sums_kernel(const Real* __restrict__ y, const Real* __restr
   for (int k = 0; k < K; ++k) acc[k] = 0.0;
   const double m = mu[v], gi = gain[v], w = wv[v];
   const double inv = K > 1 ? 1.0 / gi : 0.0;
-  // all of one mantissa bit pattern (all ones) is outside the theorem
-  const bool mid = mid_range(gi) && (__double_as_longlong(gi) & 0xfffffffffffffLL) != 0xfffffffffffffLL;
+  const bool mid = wide::divides(gi);
   for (int t = t0; t < t1; ++t) {
     const size_t base = (static_cast<size_t>(t) * n_theta + v) * n_rp;
     for (int r = threadIdx.x; r < n_r; r += blockDim.x) {
@@ -174,7 +158,7 @@ __global__ void view_sums_kernel(const Real* __restrict__ y, const Real* __restr
         acc[0] += ev * ev;
       } else {
         const double yv = y[base + r];
-        const double yh = div_by(yv - ev - m, gi, inv, mid);
+        const double yh = wide::div_by(yv - ev - m, gi, inv, mid);
         acc[0] += yv * w;
         acc[1] += w;
         acc[2] += yh * w;

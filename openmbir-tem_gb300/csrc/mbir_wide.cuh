@@ -184,5 +184,24 @@ __device__ __forceinline__ double block_sums(const double (&acc)[K]) {
   return s;
 }
 
+// x / g, correctly rounded, from inv = rn(1 / g): one refinement makes the quotient faithful, a
+// second one correctly rounded (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990), while neither the quotient nor the residuals leave the normal
+// range: here both magnitudes within 2^-400 to 2^401, the quotient then within 2^-801 to 2^801.
+__device__ __forceinline__ bool mid_range(double x) {
+  const unsigned e = (static_cast<unsigned>(__double2hiint(x)) >> 20) & 0x7ffu;
+  return e - 623u < 801u;
+}
+// whether div_by may use g's inverse (a mantissa of ones only is outside the theorem)
+__device__ __forceinline__ bool divides(double g) {
+  return mid_range(g) && (__double_as_longlong(g) & 0xfffffffffffffLL) != 0xfffffffffffffLL;
+}
+__device__ __forceinline__ double div_by(double x, double g, double inv, bool mid) {
+  if (!mid || !mid_range(x)) return x / g;
+  double q = __dmul_rn(x, inv);
+  q = fma(fma(-q, g, x), inv, q);
+  return fma(fma(-q, g, x), inv, q);
+}
+
 }  // namespace wide
 }  // namespace mbir

@@ -7,6 +7,7 @@
 
 #include "mbir_engine.h"
 #include "mbir_internal.h"
+#include "mbir_wide.cuh"
 
 using namespace mbir;
 
@@ -63,6 +64,11 @@ struct Sino {
     b.n_t = n_t;
   }
 };
+
+__global__ void div_by_kernel(const double* x, const double* g, double* q, int n) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    q[i] = wide::div_by(x[i], g[i], 1.0 / g[i], wide::divides(g[i]));
+}
 
 int done() { return cudaDeviceSynchronize() == cudaSuccess ? 0 : -3; }
 
@@ -149,6 +155,15 @@ int t_rebuild_error(const float* y, float* e, const double* mu_old, const double
                                       nullptr);
   if (rc || done()) return rc ? rc : -3;
   de.get(e);
+  return 0;
+}
+
+// q = x / g by the view sums' division
+int t_div_by(const double* x, const double* g, double* q, int n) {
+  Dev<double> dx(x, n), dg(g, n), dq(nullptr, n);
+  div_by_kernel<<<152, 256>>>(dx.d, dg.d, dq.d, n);
+  if (cudaGetLastError() != cudaSuccess || done()) return -3;
+  dq.get(q, n);
   return 0;
 }
 
