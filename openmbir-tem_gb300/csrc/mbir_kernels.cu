@@ -336,7 +336,8 @@ __global__ void __launch_bounds__(256)
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
-// One warp per column (the sums are of 2^-32 multiples below 2^21 or counts: exact in any order)
+// One warp per column: 32 rows loaded at a time, added in row order (a sum of |x| over millions of
+// voxels needs more than 53 bits of 2^-32, so the order shows in its last ones)
 __global__ void reduce_rows_kernel(const double* __restrict__ in, int n_rows, int n_cols,
                                    double* __restrict__ out, const int* __restrict__ err,
                                    const int* __restrict__ count) {
@@ -349,8 +350,16 @@ __global__ void reduce_rows_kernel(const double* __restrict__ in, int n_rows, in
   const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (c >= n_cols) return;
   double s = 0.0;
-  for (int r = lane; r < n_rows; r += 32) s += in[static_cast<size_t>(r) * n_cols + c];
-  s = warp_sum(s);
+  for (int r0 = 0; r0 < n_rows; r0 += 32) {
+    const double v = r0 + lane < n_rows ? in[static_cast<size_t>(r0 + lane) * n_cols + c] : 0.0;
+    const int n = min(32, n_rows - r0);
+    if (n == 32) {
+#pragma unroll
+      for (int k = 0; k < 32; ++k) s += __shfl_sync(kFull, v, k);
+    } else {
+      for (int k = 0; k < n; ++k) s += __shfl_sync(kFull, v, k);
+    }
+  }
   if (lane == 0) out[c] = s;
 }
 
