@@ -69,16 +69,31 @@ int Batch::ensure_resources() {
     ev0_ = a;
     ev1_ = b;
   }
+  const int device = device_;
+  auto alloc = [device](auto** p, size_t bytes) {
+    return device_malloc(reinterpret_cast<void**>(p), bytes, device);
+  };
   const size_t n = eng_.size();
   if (n > cap_series_) {
     if (d_series_) cudaFree(d_series_);
     if (d_ctr_) cudaFree(d_ctr_);
     if (d_st4_) cudaFree(d_st4_);
     cap_series_ = std::max<size_t>(n, 64);
-    if (cudaMalloc(&d_series_, sizeof(SweepArgs) * cap_series_) != cudaSuccess ||
-        cudaMalloc(&d_ctr_, sizeof(int) * (kShapes + 2 * cap_series_)) != cudaSuccess ||
-        cudaMalloc(&d_st4_, sizeof(double) * kStatSlots * cap_series_) != cudaSuccess)
+    if (alloc(&d_series_, sizeof(SweepArgs) * cap_series_) != cudaSuccess ||
+        alloc(&d_ctr_, sizeof(int) * (kShapes + 2 * cap_series_)) != cudaSuccess ||
+        alloc(&d_st4_, sizeof(double) * kStatSlots * cap_series_) != cudaSuccess)
       return fail(MBIR_ENOMEM, "batch: device allocation");
+  }
+  size_t items = 0;
+  for (Engine* e : eng_) items += static_cast<size_t>(e->geometry().n_y);
+  if (items > cap_items_) {
+    if (d_items_) cudaFree(d_items_);
+    d_items_ = nullptr;
+    cap_items_ = 0;
+    if (alloc(&d_items_, sizeof(int2) * items * 2) != cudaSuccess)
+      return fail(MBIR_ENOMEM, "batch: item allocation");
+    cap_items_ = items * 2;
+    dirty_ = true;
   }
   return MBIR_OK;
 }
@@ -132,12 +147,6 @@ int Batch::build_items(const std::vector<SweepArgs>& args) {
       }
     group_cnt_[g] = static_cast<int>(items_.size()) - group_off_[g];
   }
-  if (items_.size() > cap_items_) {
-    if (d_items_) cudaFree(d_items_);
-    cap_items_ = items_.size() * 2;
-    if (cudaMalloc(&d_items_, sizeof(int2) * cap_items_) != cudaSuccess)
-      return fail(MBIR_ENOMEM, "batch: item allocation");
-  }
   cudaMemcpy(d_items_, items_.data(), sizeof(int2) * items_.size(), cudaMemcpyHostToDevice);
   return MBIR_OK;
 }
@@ -164,6 +173,9 @@ int Batch::sweep(const std::vector<std::pair<int, int>>& iters, double* stats) {
   const bool two = threads == 256;
   const size_t stage_cap = two ? static_cast<size_t>(std::min(max_optin, per_sm / 2 - 1024)) - 2048
                                : static_cast<size_t>(max_optin) - 2048;
+  // the engines' tables until the launches that read them are queued (nothing below allocates)
+  std::vector<std::unique_lock<std::mutex>> tables;
+  for (Engine* e : eng_) tables.push_back(e->hold_table());
   // per-engine set-up (row order, bright-field list, active mask, level schedule) side by side
   const std::vector<int> rcs = parallel_for(n, device_, [&](int i) {
     const int outer = iters.empty() ? 0 : iters[i].first;
@@ -242,6 +254,7 @@ int Batch::sweep(const std::vector<std::pair<int, int>>& iters, double* stats) {
   }
   for (size_t k = 1; k < launch.size(); k++)
     cudaStreamWaitEvent(s, static_cast<cudaEvent_t>(side_ev_[k - 1]), 0);
+  tables.clear();
   if (launch_rc) {
     const std::string why = cudaGetErrorString(cudaGetLastError());
     cudaStreamSynchronize(s);  // the other launches work on the engines' arrays

@@ -15,6 +15,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <sstream>
 
 #include "mbir_engine.h"
@@ -30,14 +31,15 @@ constexpr double kFilter[27] = {0.0302, 0.0370, 0.0302, 0.0370, 0.0523, 0.0370, 
                                 0.0523, 0.0370, 0.0523, 0.0370, 0.0302, 0.0370, 0.0302,
                                 0.0370, 0.0523, 0.0370, 0.0302, 0.0370, 0.0302};
 
-template <typename T>
-int dmalloc(T** p, size_t n) {
-  if (n == 0) n = 1;
-  return cudaMalloc(reinterpret_cast<void**>(p), n * sizeof(T)) == cudaSuccess ? 0 : MBIR_ENOMEM;
-}
-int dmalloc_bytes(void** p, size_t bytes) {
-  if (bytes == 0) bytes = 16;
-  return cudaMalloc(p, bytes) == cudaSuccess ? 0 : MBIR_ENOMEM;
+// engines that hold an optional table; its lock is taken before any engine's table_mu_.  (Never
+// destroyed: an engine of static storage may outlive other statics.)
+struct TableHolders {
+  std::mutex mu;
+  std::set<Engine*> engines;
+};
+TableHolders& table_holders() {
+  static TableHolders* h = new TableHolders;
+  return *h;
 }
 template <typename T>
 void dfree(T*& p) {
@@ -45,6 +47,49 @@ void dfree(T*& p) {
   p = nullptr;
 }
 }  // namespace
+
+// ---- optional A-column tables -------------------------------------------------------------
+// Launches that may still read the table are queued before the engine's lock is free, and have run
+// when the device is idle.
+void Engine::free_optional_table() {
+  std::lock_guard<std::mutex> lk(table_mu_);
+  if (!table_optional_) return;
+  cudaDeviceSynchronize();
+  dfree(d_acol_);
+  table_optional_ = false;
+}
+
+void Engine::give_back_table() {
+  TableHolders& h = table_holders();
+  std::lock_guard<std::mutex> lk(h.mu);
+  if (h.engines.erase(this)) free_optional_table();
+}
+
+size_t Engine::optional_table_bytes() const {
+  std::lock_guard<std::mutex> lk(table_mu_);
+  return table_optional_ ? acol_bytes() : 0;
+}
+
+void reclaim_tables(int device) {
+  TableHolders& h = table_holders();
+  std::lock_guard<std::mutex> lk(h.mu);
+  for (auto it = h.engines.begin(); it != h.engines.end();) {
+    if ((*it)->params().device == device) {
+      (*it)->free_optional_table();
+      it = h.engines.erase(it);
+    } else {
+      ++it;
+    }
+  }
+}
+
+cudaError_t device_malloc(void** p, size_t bytes, int device) {
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  reclaim_tables(device);
+  return cudaMalloc(p, bytes);
+}
 
 // ---- MT19937 ------------------------------------------------------------------------------
 void MT19937::seed(uint32_t s) {
@@ -97,6 +142,12 @@ Engine::Engine(const mbir_params& p) : p_(p) {
 Engine::~Engine() { release(); }
 
 void Engine::release() {
+  {
+    TableHolders& h = table_holders();
+    std::lock_guard<std::mutex> lk(h.mu);
+    h.engines.erase(this);
+  }
+  table_optional_ = false;
   dfree(d_y_);
   dfree(d_e_);
   dfree(d_yest_);
@@ -651,6 +702,13 @@ int Engine::alloc_device() {
     smem_bytes_ = sweep_smem_bytes(g.n_theta, g.n_x, 0, t_rows_, bins_, fp64_, 0);
     smem_sched_bytes_ = sweep_smem_bytes(g.n_theta, g.n_x, 0, t_rows_, bins_, fp64_, 0, true);
   }
+  const int device = p_.device;
+  auto dmalloc_bytes = [device](void** p, size_t bytes) {
+    return device_malloc(p, bytes ? bytes : 16, device) == cudaSuccess ? 0 : MBIR_ENOMEM;
+  };
+  auto dmalloc = [&](auto** p, size_t n) {
+    return dmalloc_bytes(reinterpret_cast<void**>(p), n * sizeof(**p));
+  };
   const size_t ns = static_cast<size_t>(g.n_t) * g.n_theta * n_rp_;
   const size_t nh = static_cast<size_t>(g.n_theta) * g.n_r * g.n_t;
   const size_t nv = static_cast<size_t>(g.n_z) * g.n_x * g.n_y;
@@ -905,7 +963,8 @@ int Engine::prepare() {
       std::unique_ptr<double[]> vol(new double[nv]);
       masked(vol.get());
       double* tmp = nullptr;
-      if (cudaMalloc(&tmp, sizeof(double) * nv) != cudaSuccess) {
+      if (device_malloc(reinterpret_cast<void**>(&tmp), sizeof(double) * nv, p_.device) !=
+          cudaSuccess) {
         cudaGetLastError();
         return fail(MBIR_ENOMEM, "volume upload: device allocation failed");
       }
@@ -1012,22 +1071,25 @@ int Engine::prepare() {
 
 // The A-column table of every voxel line (FP32, parallel order), built by the sweep's own
 // arithmetic: the sweeps and projections read it instead of computing the column at every visit.
-// It is optional: without room for it (more than a quarter of the free device memory, or a
-// server that keeps its memory for other requests) the kernels compute the columns.
+// Only scheduled bright-field calls need it to be scheduled; otherwise it is optional: an engine
+// takes no more than a sixteenth of the free device memory for it, a server none that its requests'
+// own arrays need, and an allocation that fails elsewhere has it back (device_malloc).  Without it
+// the kernels compute the columns.
 int Engine::build_acol() {
   if (fp64_ || p_.order_mode != MBIR_ORDER_PARALLEL) return MBIR_OK;
   const bool scheduled = bf_ && p_.nhicd && p_.call_schedule != 1;
   const Geometry& g = g_;
   const size_t bytes = acol_bytes();
   size_t free_b = 0, total_b = 0;
-  if (!scheduled) {  // scheduled calls need the table to be scheduled
+  if (!scheduled) {
     if (!use_table_ || nb_ != 3 || !one_row_) return MBIR_OK;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4) {
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 16) {
       cudaGetLastError();
       return MBIR_OK;
     }
   }
-  if (cudaMalloc(&d_acol_, bytes) != cudaSuccess) {
+  void** const p = reinterpret_cast<void**>(&d_acol_);
+  if ((scheduled ? device_malloc(p, bytes, p_.device) : cudaMalloc(p, bytes)) != cudaSuccess) {
     cudaGetLastError();
     d_acol_ = nullptr;
     return MBIR_OK;
@@ -1035,7 +1097,14 @@ int Engine::build_acol() {
   const DevTables tab{d_H_, d_bx_, d_bxd_, d_u0_, d_bz_, d_gw_, d_tfirst_, d_tcount_, d_hval_,
                       d_lineok_};
   const int rc = launch_acol_f32(dg_, tab, nb_, d_acol_, static_cast<cudaStream_t>(stream_));
-  return rc ? cuda_check(rc, "A-column table") : MBIR_OK;
+  if (rc) return cuda_check(rc, "A-column table");
+  if (!scheduled) {
+    TableHolders& h = table_holders();
+    std::lock_guard<std::mutex> lk(h.mu);
+    h.engines.insert(this);
+    table_optional_ = true;
+  }
+  return MBIR_OK;
 }
 
 size_t Engine::acol_bytes() const {
@@ -1118,6 +1187,7 @@ int Engine::forward_project() {
   a.shape = shape_;
   a.stats = nullptr;
   a.err = d_err_;
+  auto table = hold_table();
   table_args(a);
   const size_t smem = plan_walk(a);
   for (int colour = 0; colour < 2; colour++) {
@@ -1127,6 +1197,7 @@ int Engine::forward_project() {
     int rc = launch_sweep(a, nb_, smem, s);
     if (rc) return cuda_check(rc, "forward projection launch");
   }
+  table.unlock();
   int rc;
   if (bright_field_assisted()) {
     // scaled error e / m and per-entry weights m^2 w (mbir_bfassist.cu)
@@ -1234,6 +1305,7 @@ int Engine::sweep(int outer, int inner, double* stats4) {
     a.n_rs = stage_ ? n_rs_ : 0;
     a.shape = shape_;
     a.err = d_err_;
+    const auto table = hold_table();
     table_args(a);
     if (bright_field_assisted()) {
       a.bf = 1;
@@ -1990,9 +2062,10 @@ int Engine::autotune_shape() {
   const size_t nsb = bf_ ? static_cast<size_t>(g.n_t) * g.n_theta * n_sp_ : 0;
   const size_t nl = static_cast<size_t>(g.n_z) * g.n_x;
   void *sx = nullptr, *se = nullptr, *ss = nullptr, *sm = nullptr;
-  if (cudaMalloc(&sx, nvb) != cudaSuccess || cudaMalloc(&se, neb) != cudaSuccess ||
-      (nsb && cudaMalloc(&ss, nsb) != cudaSuccess) ||
-      (bf_ && cudaMalloc(&sm, nl * sizeof(unsigned long long)) != cudaSuccess)) {
+  if (device_malloc(&sx, nvb, p_.device) != cudaSuccess ||
+      device_malloc(&se, neb, p_.device) != cudaSuccess ||
+      (nsb && device_malloc(&ss, nsb, p_.device) != cudaSuccess) ||
+      (bf_ && device_malloc(&sm, nl * sizeof(unsigned long long), p_.device) != cudaSuccess)) {
     cudaFree(sx);
     cudaFree(se);
     cudaFree(ss);
@@ -2025,6 +2098,7 @@ int Engine::autotune_shape() {
   a.smem_rows = stage_ ? 1 : 0;
   a.n_rs = stage_ ? n_rs_ : 0;
   a.err = d_err_;
+  auto table = hold_table();
   table_args(a);
   if (bf_) {
     a.bf = 1;
@@ -2068,6 +2142,7 @@ int Engine::autotune_shape() {
       best = sh;
     }
   }
+  table.unlock();
   cudaFree(sx);
   cudaFree(se);
   cudaFree(ss);

@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <string>
 #include <memory>
+#include <mutex>
 #include <thread>
 #include <utility>
 #include <vector>
@@ -75,6 +76,12 @@ class MT19937 {
 
 // visit order of UpdateYSlice::execute (HAADF_ReconstructionEngine_UpdateVoxels.cpp:151-241)
 void reference_visit_order(uint32_t seed, int n_z, int n_x, std::vector<int32_t>& out);
+
+// cudaMalloc.  When the device is out of memory, the optional A-column tables of its engines are
+// given back (reclaim_tables) and the allocation is tried once more, so that no allocation fails
+// for a table that only makes another engine's sweeps faster.
+cudaError_t device_malloc(void** p, size_t bytes, int device);
+void reclaim_tables(int device);
 
 // A host volume [z][x][y] whose values are all written by whoever sizes it
 using HostVolume = std::vector<double, UninitAlloc<double>>;
@@ -180,8 +187,15 @@ class Engine {
   double* sweep_stats() const { return d_stat4_; }
   int* error_word() const { return d_err_; }
   int nb() const { return nb_; }
-  // whether prepare may build the A-column table where it is optional (build_acol), and its size
+  // whether prepare may build the A-column table where it is optional (build_acol); the bytes of
+  // such a table; to give it back (the sweeps then compute the columns: the same bits)
   void allow_table(bool on) { use_table_ = on; }
+  size_t optional_table_bytes() const;
+  void give_back_table();
+  // held from the reading of the table's pointer until the launches that use it are queued
+  std::unique_lock<std::mutex> hold_table() const {
+    return std::unique_lock<std::mutex>(table_mu_);
+  }
   bool fp64() const { return fp64_ != 0; }
   const mbir_params& params() const { return p_; }
   int state() const { return state_; }
@@ -202,6 +216,8 @@ class Engine {
   int bf_roi_sum(int kind, double* out);
   int bf_prepare_schedule();                      // A-column table for level-scheduled calls
   int build_acol();
+  void free_optional_table();
+  friend void reclaim_tables(int device);
   size_t acol_bytes() const;
   void table_args(SweepArgs& a) const;
   int host_footprint_bins();                      // acol_lo_, acol_mask_ (once, on demand)
@@ -271,6 +287,8 @@ class Engine {
   size_t smem_bytes_ = 0;
   size_t smem_sched_bytes_ = 0;  // scheduled bright-field calls
   bool use_table_ = true;        // build the A-column table where it is optional
+  mutable std::mutex table_mu_;  // d_acol_ while it is an optional table (table_optional_)
+  bool table_optional_ = false;
   bool one_row_ = false;         // every slice meets one detector row
   bool all_lines_ = false;       // no voxel line's A-column is empty
   bool sched_ready_ = false;     // scheduled calls: schedule storage and table in place

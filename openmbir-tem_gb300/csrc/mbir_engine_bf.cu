@@ -160,8 +160,12 @@ int Engine::bf_prepare_schedule() {
   const Geometry& g = g_;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   const size_t nl = static_cast<size_t>(g.n_z) * g.n_x;
-  if (d_acol_ == nullptr || cudaMalloc(&d_sched_, nl * sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&d_lofs_, (nl + 1) * sizeof(int)) != cudaSuccess) {
+  const int device = p_.device;
+  auto alloc = [device](auto** p, size_t bytes) {
+    return device_malloc(reinterpret_cast<void**>(p), bytes, device);
+  };
+  if (d_acol_ == nullptr || alloc(&d_sched_, nl * sizeof(int)) != cudaSuccess ||
+      alloc(&d_lofs_, (nl + 1) * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     dfree_any(d_sched_);
     dfree_any(d_lofs_);
@@ -178,17 +182,17 @@ int Engine::bf_prepare_schedule() {
     return host_footprint_bins();
   // device colour schedule: packed bins and scratch
   const size_t n_entries = nl * g.n_theta;
-  if (cudaMalloc(&d_packed_, n_entries * sizeof(int32_t)) != cudaSuccess ||
-      cudaMalloc(&d_vis_, nl * sizeof(int32_t)) != cudaSuccess ||
-      cudaMalloc(&d_conf_, 5 * nl * sizeof(unsigned)) != cudaSuccess ||
-      cudaMalloc(&d_colour_, nl * sizeof(int16_t)) != cudaSuccess ||
-      cudaMalloc(&d_bin_used_, static_cast<size_t>(g.n_theta) * g.n_r * cwords_ * 8) !=
+  if (alloc(&d_packed_, n_entries * sizeof(int32_t)) != cudaSuccess ||
+      alloc(&d_vis_, nl * sizeof(int32_t)) != cudaSuccess ||
+      alloc(&d_conf_, 5 * nl * sizeof(unsigned)) != cudaSuccess ||
+      alloc(&d_colour_, nl * sizeof(int16_t)) != cudaSuccess ||
+      alloc(&d_bin_used_, static_cast<size_t>(g.n_theta) * g.n_r * cwords_ * 8) !=
           cudaSuccess ||
-      cudaMalloc(&d_line_used_, nl * cwords_ * 8) != cudaSuccess ||
-      cudaMalloc(&d_sched_count_, 2 * sizeof(int32_t)) != cudaSuccess ||
-      cudaMalloc(&d_hc_lines_, nl * sizeof(int32_t)) != cudaSuccess ||
-      cudaMalloc(&d_hc_lofs_, kNumHomogeneous * lofs_cap() * sizeof(int32_t)) != cudaSuccess ||
-      cudaMalloc(&d_hc_count_, kNumHomogeneous * 2 * sizeof(int32_t)) != cudaSuccess) {
+      alloc(&d_line_used_, nl * cwords_ * 8) != cudaSuccess ||
+      alloc(&d_sched_count_, 2 * sizeof(int32_t)) != cudaSuccess ||
+      alloc(&d_hc_lines_, nl * sizeof(int32_t)) != cudaSuccess ||
+      alloc(&d_hc_lofs_, kNumHomogeneous * lofs_cap() * sizeof(int32_t)) != cudaSuccess ||
+      alloc(&d_hc_count_, kNumHomogeneous * 2 * sizeof(int32_t)) != cudaSuccess) {
     cudaGetLastError();
     dfree_any(d_packed_);
     dfree_any(d_vis_);
@@ -204,8 +208,8 @@ int Engine::bf_prepare_schedule() {
   }
   // scratch of the multi-CTA colouring (without it the one-CTA form runs)
   const size_t nblk = (nl + 30) / 31;
-  if (cudaMalloc(&d_cfsets_, nblk * 31 * cwords_ * 8) != cudaSuccess ||
-      cudaMalloc(&d_cflags_, (3 * nblk + 1) * sizeof(int)) != cudaSuccess) {
+  if (alloc(&d_cfsets_, nblk * 31 * cwords_ * 8) != cudaSuccess ||
+      alloc(&d_cflags_, (3 * nblk + 1) * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     dfree_any(d_cfsets_);
     dfree_any(d_cflags_);
@@ -213,9 +217,9 @@ int Engine::bf_prepare_schedule() {
   hc_valid_.assign(kNumHomogeneous, 0);
   hc_start_.assign(kNumHomogeneous, 0);
   // the sub-lists on the device (without them each call's lines come from the host)
-  if (cudaMalloc(&d_slot_, nl) != cudaSuccess ||
-      cudaMalloc(&d_hvis_, nl * sizeof(int32_t)) != cudaSuccess ||
-      cudaMalloc(&d_nvis_, sizeof(int32_t)) != cudaSuccess) {
+  if (alloc(&d_slot_, nl) != cudaSuccess ||
+      alloc(&d_hvis_, nl * sizeof(int32_t)) != cudaSuccess ||
+      alloc(&d_nvis_, sizeof(int32_t)) != cudaSuccess) {
     cudaGetLastError();
     dfree_any(d_slot_);
     dfree_any(d_hvis_);
@@ -625,6 +629,7 @@ int Engine::bf_call(int outer, int inner, double* st4) {
   } else {
     SweepArgs a{};
     size_t smem = 0;
+    const auto table = hold_table();
     if ((rc = bf_parallel_args(iter_nonzero, bfa, &a, &smem))) return rc;
     const int n0 = (g.n_y + 1) / 2;
     cudaEventRecord(static_cast<cudaEvent_t>(ev2_), s);

@@ -88,11 +88,16 @@ int Engine::sweep_colour(int colour, int outer, int inner, double* st4) {
   a.n_rs = stage_ ? n_rs_ : 0;
   a.shape = shape_;
   a.err = d_err_;
-  table_args(a);
-  size_t smem = plan_walk(a);
+  const auto table = hold_table();
+  size_t smem = 0;
   if (bf_) {
     a = slab_args_;
     smem = slab_smem_;
+  }
+  // (a call that is not scheduled was opened when the table may have been another)
+  if (a.sched_lines == nullptr) {
+    table_args(a);
+    smem = plan_walk(a);
   }
   a.colour = colour;
   a.y_first = first;
@@ -242,7 +247,10 @@ int Engine::bf_slab_begin(int outer, int inner) {
   int rc = bf_call_begin(outer, inner, &bfa);
   if (rc) return rc;
   const int iter_nonzero = (inner > 0 || outer > 0) ? 1 : 0;
-  if ((rc = bf_parallel_args(iter_nonzero, bfa, &slab_args_, &slab_smem_))) return rc;
+  {
+    const auto table = hold_table();
+    if ((rc = bf_parallel_args(iter_nonzero, bfa, &slab_args_, &slab_smem_))) return rc;
+  }
   slab_call_open_ = true;
   outer_ = outer;
   inner_ = inner;

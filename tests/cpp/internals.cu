@@ -167,6 +167,19 @@ int t_div_by(const double* x, const double* g, double* q, int n) {
   return 0;
 }
 
+// The engine's optional A-column table; all of a device's given back; an allocation that no device
+// has room for
+long t_optional_table_bytes(void* engine) {
+  return static_cast<long>((*static_cast<Engine**>(engine))->optional_table_bytes());
+}
+void t_reclaim_tables(int device) { reclaim_tables(device); }
+int t_huge_allocation_fails(int device) {
+  void* p = nullptr;
+  const bool failed = device_malloc(&p, size_t{1} << 50, device) == cudaErrorMemoryAllocation;
+  cudaGetLastError();
+  return failed && p == nullptr ? 1 : 0;
+}
+
 int t_reduce_stats(const double* in, int n_rows, int n_cols, double* out) {
   Dev<double> d(in, static_cast<size_t>(n_rows) * n_cols), o(nullptr, n_cols + 2);
   const int rc = launch_reduce_stats(d.d, n_rows, n_cols, o.d, nullptr);
