@@ -92,10 +92,11 @@ size_t Server::estimate_bytes(const Request& r) const {
   return rb * (3 * sino + vox) + host_layout + bf + (1u << 20);
 }
 
-// The A-column table of a HAADF request (Engine::build_acol).  It only makes the sweeps faster,
-// so no request is refused for it.
+// The optional A-column table of a request (Engine::build_acol; estimate_bytes has that of scheduled
+// calls).  It only makes the sweeps faster, so no request is refused for it.
 size_t Server::table_bytes(const Request& r) const {
-  if (r.params.modality == MBIR_MODALITY_BF) return 0;
+  if (r.params.modality == MBIR_MODALITY_BF && r.params.nhicd && r.params.call_schedule != 1)
+    return 0;
   return static_cast<size_t>(r.dims[0]) * r.dims[1] * r.n_theta * 16;
 }
 
@@ -148,12 +149,14 @@ int Server::admit_locked(std::vector<Request*>& admitted) {
     Request* r = queue_.front();
     if (used_ + tables_ + static_cast<int64_t>(r->bytes) > budget_) break;  // arrival order: no overtaking
     queue_.pop_front();
-    // tables take at most half of the budget, and none that a queued request's own arrays need
+    // a table is no larger than the request's own arrays; tables take at most half of the budget,
+    // and none that a queued request's own arrays need
     const size_t table = table_bytes(*r);
     int64_t queued = 0;
     for (const Request* q : queue_) queued += static_cast<int64_t>(q->bytes);
     const int64_t with = used_ + tables_ + static_cast<int64_t>(r->bytes + table);
-    const bool room = with + queued <= budget_ && with <= budget_ / 2;
+    const bool room =
+        table <= r->bytes && with + queued <= budget_ && with <= budget_ / 2;
     r->engine->allow_table(room);
     r->table = room ? static_cast<int64_t>(table) : 0;
     tables_ += r->table;
@@ -162,7 +165,7 @@ int Server::admit_locked(std::vector<Request*>& admitted) {
     stats_.admitted++;
     if (r->id < last_admitted_id_) stats_.admitted_out_of_order++;
     last_admitted_id_ = r->id;
-    stats_.peak_bytes = std::max(stats_.peak_bytes, used_);
+    stats_.peak_bytes = std::max(stats_.peak_bytes, used_ + tables_);
     stats_.peak_active = std::max(
         stats_.peak_active, static_cast<int32_t>(active_.size() + prepared_.size() + preparing_ +
                                                  admitted.size()));
@@ -218,6 +221,11 @@ void Server::prepare_loop() {
     lk.lock();
     preparing_ -= static_cast<int>(admitted.size());
     for (size_t k = 0; k < admitted.size(); k++) {
+      if (!rcs[k]) {  // what the engine built
+        tables_ -= admitted[k]->table;
+        admitted[k]->table = static_cast<int64_t>(admitted[k]->engine->optional_table_bytes());
+        tables_ += admitted[k]->table;
+      }
       if (rcs[k])
         retire(admitted[k], MBIR_EDEVICE, msgs[k]);
       else

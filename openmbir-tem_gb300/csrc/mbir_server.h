@@ -74,8 +74,8 @@ class Server {
   int device_;
   int64_t budget_;
   int max_active_;
-  int64_t used_ = 0;    // of the admitted requests' own arrays (peak_bytes is its maximum)
-  int64_t tables_ = 0;  // of their tables; used_ + tables_ stays within the budget
+  int64_t used_ = 0;    // of the admitted requests' own arrays
+  int64_t tables_ = 0;  // of their tables; used_ + tables_ stays within the budget (peak_bytes)
   int64_t last_admitted_id_ = 0;
   int64_t next_id_ = 1;
   mutable std::mutex mu_;

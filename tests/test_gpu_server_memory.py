@@ -1,0 +1,77 @@
+"""A server's memory account with the requests' optional A-column tables."""
+import time
+
+import numpy as np
+import pytest
+
+from conftest import bf_case, bf_params, haadf_params
+from test_gpu_table import series
+
+pytestmark = pytest.mark.gpu
+
+
+def haadf(mbir, n_r=40, n_t=64, views=41):
+    y, ang, th = series(n_r, n_t, 12, views)
+    return haadf_params(mbir, th), y, ang
+
+
+def bright_field(mbir, **kw):
+    y, ang, th = bf_case(n_r=48, n_t=40)
+    return bf_params(mbir, th, **kw), y, ang
+
+
+def dims(mbir, req):
+    p, y, ang = req
+    with mbir.Engine(p) as e:
+        e.set_sinogram(y, ang)
+        return e.dims()[:3]
+
+
+def own_bytes(mbir, req):
+    """The footprint without the table: the peak of a server whose budget has no room for one."""
+    lo, hi = 1 << 20, 1 << 30
+    p, y, ang = req
+    while hi - lo > 1:  # the smallest budget that takes the request
+        mid = (lo + hi) // 2
+        with mbir.Server(0, mid, 1) as s:
+            try:
+                s.wait(s.submit(p, y, ang, max_outer=1, tol=0.0))
+                hi = mid
+            except mbir.MbirError:
+                lo = mid
+    return hi
+
+
+def peak(mbir, req, budget):
+    p, y, ang = req
+    with mbir.Server(0, budget, 1) as s:
+        s.wait(s.submit(p, y, ang, max_outer=1, tol=0.0))
+        return s.stats().peak_bytes
+
+
+@pytest.mark.parametrize("kind", ["haadf", "bf-no-nhicd", "bf-row-walk", "bf-scheduled"])
+def test_peak_counts_the_table(lib_built, kind):
+    """peak_bytes is the largest estimated footprint resident at one time: the request's own arrays
+    and its table, where it has one."""
+    mbir = lib_built
+    req = {"haadf": haadf, "bf-no-nhicd": lambda m: bright_field(m, nhicd=0),
+           "bf-row-walk": lambda m: bright_field(m, call_schedule=1),
+           "bf-scheduled": bright_field}[kind](mbir)
+    nz, nx, _ = dims(mbir, req)
+    table = 0 if kind == "bf-scheduled" else nz * nx * len(req[2]) * 16
+    own = own_bytes(mbir, req)
+    assert table <= own
+    assert peak(mbir, req, own) == own  # no room for a table
+    assert peak(mbir, req, 2 * (own + table) - 1) == (own if table else own)
+    assert peak(mbir, req, 2 * (own + table)) == own + table
+    assert peak(mbir, req, 0) == own + table
+
+
+def test_thin_requests_take_none(lib_built):
+    """A table larger than the request's own arrays is not built."""
+    mbir = lib_built
+    req = haadf(mbir, n_r=128, n_t=2, views=61)
+    nz, nx, _ = dims(mbir, req)
+    own = own_bytes(mbir, req)
+    assert nz * nx * 61 * 16 > own
+    assert peak(mbir, req, 0) == own
