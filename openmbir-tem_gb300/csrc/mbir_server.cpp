@@ -144,10 +144,17 @@ int64_t Server::submit(const mbir_params& p, const float* counts, const float* t
 }
 
 int Server::admit_locked(std::vector<Request*>& admitted) {
+  tables_wanted_ = 0;
   while (!queue_.empty() && static_cast<int>(active_.size() + prepared_.size() + preparing_ +
                                              admitted.size()) < max_active_) {
     Request* r = queue_.front();
-    if (used_ + tables_ + static_cast<int64_t>(r->bytes) > budget_) break;  // arrival order: no overtaking
+    const int64_t over = used_ + static_cast<int64_t>(r->bytes) - budget_;
+    if (over > 0) break;  // arrival order: no overtaking
+    if (over + tables_ > 0) {  // only tables are in its way: they go first
+      tables_wanted_ = over + tables_;
+      cv_.notify_all();
+      break;
+    }
     queue_.pop_front();
     // a table is no larger than the request's own arrays; tables take at most half of the budget,
     // and none that a queued request's own arrays need
@@ -171,6 +178,22 @@ int Server::admit_locked(std::vector<Request*>& admitted) {
                                                  admitted.size()));
   }
   return 0;
+}
+
+// The worker, between steps (mu_ held, no launch of its own in flight): tables back from the
+// requests that came last until the next arrival's own arrays have room
+void Server::give_back_tables() {
+  for (auto* list : {&prepared_, &active_})
+    for (auto it = list->rbegin(); it != list->rend() && tables_wanted_ > 0; ++it) {
+      Request* r = *it;
+      if (r->table == 0) continue;
+      r->engine->give_back_table();
+      tables_ -= r->table;
+      tables_wanted_ -= r->table;
+      r->table = 0;
+    }
+  tables_wanted_ = 0;
+  cv_.notify_all();  // the preparer admits
 }
 
 void Server::retire(Request* r, int code, const std::string& msg) {
@@ -242,6 +265,7 @@ void Server::loop() {
   for (;;) {
     cv_.wait(lk, [&] { return stop_ || !prepared_.empty() || !active_.empty(); });
     if (stop_) break;
+    if (tables_wanted_ > 0) give_back_tables();
     std::vector<Request*> joining;
     joining.swap(prepared_);
     lk.unlock();

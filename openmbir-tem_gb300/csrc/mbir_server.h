@@ -69,6 +69,7 @@ class Server {
   size_t estimate_bytes(const Request& r) const;
   size_t table_bytes(const Request& r) const;
   int admit_locked(std::vector<Request*>& admitted);
+  void give_back_tables();
   void retire(Request* r, int code, const std::string& msg);
 
   int device_;
@@ -76,6 +77,7 @@ class Server {
   int max_active_;
   int64_t used_ = 0;    // of the admitted requests' own arrays
   int64_t tables_ = 0;  // of their tables; used_ + tables_ stays within the budget (peak_bytes)
+  int64_t tables_wanted_ = 0;  // bytes of tables that keep the next arrival waiting
   int64_t last_admitted_id_ = 0;
   int64_t next_id_ = 1;
   mutable std::mutex mu_;

@@ -75,3 +75,33 @@ def test_thin_requests_take_none(lib_built):
     own = own_bytes(mbir, req)
     assert nz * nx * 61 * 16 > own
     assert peak(mbir, req, 0) == own
+
+
+def test_tables_make_way_for_an_arrival(lib_built):
+    """A request whose own arrays fit beside those of an active one joins it: the active one's table,
+    which takes the room, goes back, and its result keeps every bit."""
+    mbir = lib_built
+    first, second = haadf(mbir), haadf(mbir, n_t=96)
+    nz, nx, _ = dims(mbir, first)
+    table = nz * nx * len(first[2]) * 16
+    own1, own2 = own_bytes(mbir, first), own_bytes(mbir, second)
+    budget = own1 + own2 + table // 2
+    assert own1 + table <= budget // 2  # the first is granted its table
+    outers = 1500
+    with mbir.Server(0, own1, 1) as s:
+        rid = s.submit(*first, max_outer=outers, tol=0.0)
+        s.wait(rid)
+        want = s.result(rid)
+    with mbir.Server(0, budget, 2) as s:
+        r1 = s.submit(*first, max_outer=outers, tol=0.0)
+        t0 = time.monotonic()
+        while s.poll(r1)[0] == 0 and time.monotonic() - t0 < 60:
+            time.sleep(0.001)
+        assert s.stats().peak_bytes == own1 + table
+        r2 = s.submit(*second, max_outer=2, tol=0.0)
+        s.wait(r2)
+        assert s.poll(r1)[0] == 1  # the first still runs
+        st = s.stats()
+        assert st.peak_active == 2 and st.peak_bytes <= budget
+        s.wait(r1)
+        assert np.array_equal(s.result(r1), want)
