@@ -2033,7 +2033,9 @@ int Engine::write_outputs(const char* dir, const char* mrc_path, const char* vtk
 // line, the current state) on a snapshot of the volume, error sinogram and selector; the state
 // is restored after every trial and the fastest candidate is kept.  Choices are cached per
 // (views, x, z, y, footprint bins, modality, staging) for the life of the process, so engines of
-// the same geometry tune once.
+// the same geometry tune once.  The A-column table is not part of the key although it changes the
+// times: whether an engine has one depends on the memory left, the shape decides in which order its
+// sums round, and a series must give the same bits in every request.
 namespace {
 std::mutex g_tune_mu;
 std::map<std::vector<int>, int> g_tune_cache;

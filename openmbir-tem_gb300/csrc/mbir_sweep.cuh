@@ -1585,7 +1585,8 @@ int launch_slices(const SweepArgs& a, size_t smem, int threads, cudaStream_t s) 
   return ok_or(cudaGetLastError());
 }
 
-// The launch with `ctas` CTAs per slice; 1 when the device does not hold that many clusters at once
+// The launch with `ctas` CTAs per slice.  Returns 0 without a launch (`launched` false) when the
+// device does not hold that many clusters at once or the layout does not fit.
 template <auto k>
 int launch_clusters(const SweepArgs& a, size_t smem, int ctas, cudaStream_t s, bool& launched) {
   launched = false;

@@ -652,7 +652,10 @@ __device__ __forceinline__ void walk_rows(const SweepArgs& A, const TableLayout&
     // period's prefix-OR, and the period's last voxel also follows the next period's first one.
     // `dense`: so many candidates (N) that neighbouring classes practically always have some
     // within S of each other (N / S per class: 2 N^2 / (S n_x) close pairs expected), so that the
-    // search for classes to merge is left out.
+    // search for classes to merge is left out.  (Counted are the threads that saw one, N itself
+    // while n_x is at most the CTA's threads.  In longer rows a thread may stand for several; the
+    // line at sqrt(S n_x / 2), 78 of 4000 voxels at S = 3, is far below the threads, so that only
+    // rows with that few candidates can fall on either side.  Results do not depend on it.)
     int any_cand = 0;
     bool dense = true;
     if (kProject || !zs_on) {
@@ -1030,7 +1033,11 @@ int launch_table_pick(const SweepArgs& a, size_t smem, cudaStream_t s) {
 }
 
 // The persistent batched sweep (batch_sweep_kernel) of table-driven series, staged or not in
-// separate launches: with both forms in one kernel it spilled 200 to 900 bytes a thread.
+// separate launches.  It still spills where the same step launched alone does not (0 to 52 bytes of
+// stores a thread up to 160 views): the arguments come from a shared copy instead of the constant
+// bank, and bright field holds the row walk and the scheduled call in one kernel.  Bytes of spill
+// stores staged / in HBM: bright field 16 x 4 356 / 388, 32 x 2 48 / 28, 32 x 3 164 / 148, 32 x 5
+// 480 / 508; HAADF 108 / 96, 8 / 0, 16 / 4, 120 / 100.
 template <int G, int VPL, bool STAGE, bool BF>
 __global__ void __launch_bounds__(kWarps * 32, 1) batch_table_kernel(BatchArgs B) {
   batch_items(B, [](const SweepArgs& sA, int y, unsigned char* smem, uint32_t& phase,
