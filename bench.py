@@ -712,13 +712,14 @@ def main():
     peak, peak_kind = load_peaks()
     achieved = bytes_step / (kernel_ms_step / 1e3) / 1e9
     launches = calls_per_step * 3  # two colour launches + one stats reduction per call
-    traffic = None
+    traffic, kernel = None, "table_kernel"
     tp = os.path.join(ROOT, "profiles", "icd_sweep_traffic.json")
     if os.path.exists(tp):
         try:
             with open(tp) as f:
                 ent = json.load(f).get(args.workload)
             traffic = ent.get("bytes_per_launch") if isinstance(ent, dict) else ent
+            kernel = ent.get("kernel", kernel) if isinstance(ent, dict) else kernel
         except Exception:
             traffic = None
 
@@ -747,7 +748,7 @@ def main():
                         "traffic_unit": "bytes per colour launch (ncu capture)",
                         "bytes_model": ("13*F*L+8" if bf else "8*F*L+8") +
                                        " per updated voxel, F=A-column nnz, L=t rows",
-                        "kernel": "sweep_kernel (two colour launches per call)",
+                        "kernel": kernel + " (two colour launches per call)",
                         "kernel_ms_per_launch": kernel_ms_step / (2 * calls_per_step)},
            "clocks": clk.summary()}
 
