@@ -261,10 +261,8 @@ __global__ void __launch_bounds__(256)
             if constexpr (KIND == kOffsetSums) {
               sum[0].add(wide::two_prod(ev[j], wv[j]));
               sum[1].add(wv[j]);
-            } else {  // e^2 w exactly: the two parts of e^2 times w, two pairs
-              const wide::F2 q = wide::two_prod(ev[j], ev[j]);
-              sum[0].add(wide::two_prod(q.hi, wv[j]));
-              sum[0].add(wide::two_prod(q.lo, wv[j]));
+            } else {
+              sum[0].add_square_times(ev[j], wv[j]);
             }
           } else {
             rejected = true;

@@ -79,6 +79,13 @@ struct WideSum {
     s1 = c.hi;
     s2 = __fadd_rn(s2, __fadd_rn(b.lo, c.lo));
   }
+  // e^2 w, exact to the sum's own rounding: both parts of e^2 times w, the two low ends combined
+  __device__ __forceinline__ void add_square_times(float e, float w) {
+    const F2 q = two_prod(e, e), p = two_prod(q.hi, w), t = two_prod(q.lo, w);
+    const F2 r = two_sum(p.lo, t.hi);
+    add(F2{p.hi, r.hi});
+    s2 = __fadd_rn(s2, __fadd_rn(r.lo, t.lo));
+  }
   __device__ __forceinline__ double value() const {
     return static_cast<double>(s0) + (static_cast<double>(s1) + static_cast<double>(s2));
   }
