@@ -23,6 +23,13 @@ namespace mbir {
 namespace {
 constexpr int kTableSlices = 16;  // fewest slices of a request with an optional table
 
+// voxel / detector pixel size of the request's level
+int level_factor(const mbir_params& p) {
+  const int levels = std::max(1, p.num_resolutions);
+  const int lvl = (p.level < 0 || p.level >= levels) ? levels - 1 : p.level;
+  return (1 << (levels - 1 - lvl)) * std::max(1, p.final_resolution);
+}
+
 double now_s() {
   return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
@@ -77,11 +84,7 @@ size_t Server::estimate_bytes(const Request& r) const {
       // scheduled NHICD calls (Engine::bf_prepare_schedule): the A-column table of every line,
       // [lines][n_theta][acol_width(nb)] float4 with nb = 2 * (voxel / detector size) + 1, the
       // schedule, and the device colouring's packed bins, conflict words and colour planes
-      const int levels = std::max(1, r.params.num_resolutions);
-      const int lvl = (r.params.level < 0 || r.params.level >= levels) ? levels - 1
-                                                                       : r.params.level;
-      const int factor = (1 << (levels - 1 - lvl)) * std::max(1, r.params.final_resolution);
-      const size_t acol_w = static_cast<size_t>(2 * factor + 1 + 4) / 4;
+      const size_t acol_w = static_cast<size_t>(2 * level_factor(r.params) + 1 + 4) / 4;
       const size_t entries = lines * r.n_theta;
       const size_t words = 16;  // 64-bit colour words per bin / line (1024 colours)
       const size_t blocks = (lines + 30) / 31;  // 31-line blocks of the multi-CTA colouring
@@ -104,7 +107,7 @@ size_t Server::estimate_bytes(const Request& r) const {
 size_t Server::table_bytes(const Request& r) const {
   if (r.params.modality == MBIR_MODALITY_BF && r.params.nhicd && r.params.call_schedule != 1)
     return 0;
-  if (r.dims[2] < kTableSlices) return 0;
+  if (r.dims[2] < kTableSlices || level_factor(r.params) != 1) return 0;
   return static_cast<size_t>(r.dims[0]) * r.dims[1] * r.n_theta * 16;
 }
 

@@ -10,9 +10,9 @@ from test_gpu_table import series
 pytestmark = pytest.mark.gpu
 
 
-def haadf(mbir, n_r=40, n_t=64, views=41):
+def haadf(mbir, n_r=40, n_t=64, views=41, **kw):
     y, ang, th = series(n_r, n_t, 12, views)
-    return haadf_params(mbir, th), y, ang
+    return haadf_params(mbir, th, **kw), y, ang
 
 
 def bright_field(mbir, **kw):
@@ -49,16 +49,17 @@ def peak(mbir, req, budget):
         return s.stats().peak_bytes
 
 
-@pytest.mark.parametrize("kind", ["haadf", "bf-no-nhicd", "bf-row-walk", "bf-scheduled"])
+@pytest.mark.parametrize("kind", ["haadf", "bf-no-nhicd", "bf-row-walk", "bf-scheduled", "coarse"])
 def test_peak_counts_the_table(lib_built, kind):
     """peak_bytes is the largest estimated footprint resident at one time: the request's own arrays
     and its table, where it has one."""
     mbir = lib_built
     req = {"haadf": haadf, "bf-no-nhicd": lambda m: bright_field(m, nhicd=0),
            "bf-row-walk": lambda m: bright_field(m, call_schedule=1),
-           "bf-scheduled": bright_field}[kind](mbir)
+           "bf-scheduled": bright_field,
+           "coarse": lambda m: haadf(m, num_resolutions=2, level=0)}[kind](mbir)
     nz, nx, _ = dims(mbir, req)
-    table = 0 if kind == "bf-scheduled" else nz * nx * len(req[2]) * 16
+    table = 0 if kind in ("bf-scheduled", "coarse") else nz * nx * len(req[2]) * 16
     own = own_bytes(mbir, req)
     assert peak(mbir, req, own) == own  # no room for a table
     assert peak(mbir, req, 2 * (own + table) - 1) == (own if table else own)
